@@ -195,7 +195,7 @@ class HistoPyramid:
         return out
 
     def classify_path(self) -> int:
-        """1: TMA column kernel, 0: generic per-block kernel (last build)."""
+        """1: TMA column kernel, 0: a direct-load kernel (last build)."""
         p = C.c_int(-1)
         _check(lib().HPMCgetClassifyPath(self.ptr, C.byref(p)), "HPMCgetClassifyPath")
         return int(p.value)

@@ -176,7 +176,7 @@ int bind_field(HPMCHistoPyramid* h) {
     V.slice_pitch = (long long)(sp / es);
     V.idx32 = (V.slice_pitch * ((long long)h->lattice[2] + 1) < (1ll << 31)) ? 1 : 0;
     // TMA column path: column layout, 16-byte aligned base and pitches
-    // (scalar fields only: a float4 field takes the generic classifier)
+    // (scalar fields only: a float4 field takes the direct column classifier)
     h->have_tmap = V.column_layout && f.type != HPMC_SCALAR_F32X4 && ((uintptr_t)f.ptr % 16 == 0) &&
                    rp % 16 == 0 && sp % 16 == 0 &&
                    hpmc::host::encode_column_map(&h->tmap, f.ptr, f.type, h->lattice, rp, sp);
@@ -494,7 +494,7 @@ void HPMCbuildHistopyramid(HPMCHistoPyramid* h, GLfloat threshold) {
     const int max_ctas = h->constants->num_sms * 16;
     cudaError_t e;
     if (V.ftype == hpmc::kFieldUser) {
-        // the caller's instantiation of the generic classifier (include/hpmc_functor.cuh)
+        // the caller's instantiation of the direct classifiers (include/hpmc_functor.cuh)
         const int grid = (int)std::min<long long>(V.nblocks, (long long)max_ctas);
         e = h->user_ops.classify(&V, grid, h->stream) == HPMC_OK ? cudaSuccess : cudaErrorLaunchFailure;
     } else {

@@ -19,28 +19,19 @@
 #include "hpmc_fetch.cuh"
 #include "hpmc_kernels.h"
 #include "hpmc_tma.cuh"
-#include "hpmc_classify_core.cuh"
+#include "hpmc_column_core.cuh"
 
 namespace hpmc {
 
 // ---------------------------------------------------------------------------
-// Column classification: a column = one 32x32 cell footprint of the slice
-// tiles x column_slices slices, streamed through a TMA ring of 8-layer
-// sample boxes (each sample leaves HBM once; halo rows/columns are shared
-// with neighbouring columns through L2).  The single-volume kernel is
-// persistent (columns from a device queue); the batched one takes one column
-// brick per CTA.
-//
-// Per layer, every warp turns rows of samples into bits (f < iso) with one
-// ballot per row.  Per slice, ONE warp classifies the whole 32x32 block,
-// bit-sliced: lane y holds the 32 cells of row y as eight 32-bit words, word
-// k = bit k (dx + 2dy + 4dz) of the 32 codes.  AND/OR over the eight words
-// marks the cells that are neither all-inside nor all-outside (the only ones
-// with vertices); only those go through the count table.  The warp sum is the
-// block's level-5 entry; non-empty blocks also store their 1024 codes in
-// Morton order and each 32-cell tile's active mask and vertex count in their
-// arena slot (1.25 KiB), from which a traversal warp builds the block's
-// active-cell list when it enters the block.
+// TMA column classification (hpmc_column_core.cuh has the classification of a
+// box): a column's boxes stream through a TMA ring (each sample leaves HBM
+// once; halo rows/columns are shared with neighbouring columns through L2).
+// The single-volume kernel is persistent (columns from a device queue); the
+// batched one takes one column brick per CTA.  Non-empty blocks store their
+// 1024 codes in Morton order and each 32-cell tile's active mask and vertex
+// count in their arena slot (1.25 KiB), from which a traversal warp builds the
+// block's active-cell list when it enters the block.
 //
 // Measured alternatives for the list: written by the classifier (each
 // non-empty block's serial gathers stall the box barrier: +20 us at 512^3),
@@ -48,179 +39,6 @@ namespace hpmc {
 // ~500 warp instructions per list, not hidden by the 7 us reduction tree:
 // +11 us) -- both slower than one build per warp in the traversal, where the
 // latency of the list's gathers overlaps other warps' vertex work.
-namespace {
-
-template <int FT, typename T>
-__device__ __forceinline__ bool below(T v, float iso, int u8_thr) {
-    if constexpr (FT == kFieldF32)
-        return v < iso;  // strict; NaN -> false (shadergen.cpp:137-142)
-    else
-        return (int)v < u8_thr;
-}
-
-// 8x8 bit-matrix transpose: byte r bit c -> byte c bit r.
-__device__ __forceinline__ uint64_t transpose8(uint64_t x) {
-    uint64_t t;
-    t = (x ^ (x >> 7)) & 0x00AA00AA00AA00AAull;
-    x = x ^ t ^ (t << 7);
-    t = (x ^ (x >> 14)) & 0x0000CCCC0000CCCCull;
-    x = x ^ t ^ (t << 14);
-    t = (x ^ (x >> 28)) & 0x00000000F0F0F0F0ull;
-    x = x ^ t ^ (t << 28);
-    return x;
-}
-
-// Bit-sliced codes of one 32-cell row -> 32 byte codes (w[i] = cells 4i..4i+3).
-__device__ __forceinline__ void slices_to_codes(const uint32_t c[8], uint32_t w[8]) {
-#pragma unroll
-    for (int g = 0; g < 4; g++) {
-        const uint32_t sel = (uint32_t)g | ((uint32_t)(g + 4) << 4);
-        const uint32_t lo = __byte_perm(__byte_perm(c[0], c[1], sel), __byte_perm(c[2], c[3], sel), 0x5410);
-        const uint32_t hi = __byte_perm(__byte_perm(c[4], c[5], sel), __byte_perm(c[6], c[7], sel), 0x5410);
-        const uint64_t x = transpose8((uint64_t)lo | ((uint64_t)hi << 32));
-        w[2 * g] = (uint32_t)x;
-        w[2 * g + 1] = (uint32_t)(x >> 32);
-    }
-}
-
-// 16 bits -> Morton positions of an 8x2 cell tile: bit x of the low byte goes
-// to bit (x0 | x1 << 2 | x2 << 4), bit x of the high byte to that + 8.
-__device__ __forceinline__ uint32_t spread16(uint32_t t) {
-    t = (t | (t << 12)) & 0x0F0F0F0Fu;
-    return (t | (t << 2)) & 0x33333333u;
-}
-
-// One warp: classify slice z of footprint (fx, fy) from sample-bit rows of the
-// lower layer (rows_b/col_b) and the upper layer (rows_t/col_t).  Every block
-// gets its level-5 count; blocks with vertices store their codes in Morton
-// order in their slot.  full: every cell of the footprint lies inside the
-// grid (vmask is all ones in every lane).  b: the block's level-5 index,
-// column_block_index(V, z, fx, fy).
-__device__ __forceinline__ void classify_slice_warp(const Volume& V, int z, int fx, int fy, uint32_t b, int lane,
-                                                    uint32_t vmask, bool full, const uint32_t* rows_b,
-                                                    uint64_t col_b, const uint32_t* rows_t, uint64_t col_t,
-                                                    const uint8_t* s_cnt) {
-    // rows y and y+1 of both layers; bit 32 of a row (column x0+32) comes
-    // from the column word: (row >> 1) | colbit << 31 is the row shifted by one cell
-    const uint32_t cbl = (uint32_t)col_b, cbh = (uint32_t)(col_b >> 32);
-    const uint32_t ctl = (uint32_t)col_t, cth = (uint32_t)(col_t >> 32);
-    const uint32_t a0 = rows_b[lane], a1 = rows_b[lane + 1];
-    const uint32_t b0 = rows_t[lane], b1 = rows_t[lane + 1];
-    if (full && !V.codes_out) {
-        // A full block has no vertices iff its 33x33x2 samples all lie on one
-        // side of the iso-value (two samples that differ have some edge
-        // between them that differs, and every edge belongs to a cell of the
-        // block): one AND and one OR of the lane's two rows in both layers
-        // and of its two column bits, two votes.
-        const uint32_t cb = __funnelshift_r(cbl, cbh, lane) & 3u, ct = __funnelshift_r(ctl, cth, lane) & 3u;
-        const bool below_all = ((a0 & a1 & b0 & b1) == 0xffffffffu) && ((cb & ct) == 3u);
-        const bool above_all = ((a0 | a1 | b0 | b1) == 0u) && ((cb | ct) == 0u);
-        if (__all_sync(0xffffffffu, below_all) || __all_sync(0xffffffffu, above_all)) {
-            if (lane == 0) V.levels[V.level_off[kBlockLevel] + b] = 0u;
-            return;
-        }
-    }
-    uint32_t c[8];
-    c[0] = a0;                                                   // (x,   y,   z)
-    c[1] = (a0 >> 1) | (((cbl >> lane) & 1u) << 31);             // (x+1, y,   z)
-    c[2] = a1;                                                   // (x,   y+1, z)
-    c[3] = (a1 >> 1) | ((__funnelshift_rc(cbl, cbh, lane + 1) & 1u) << 31);
-    c[4] = b0;                                                   // (x,   y,   z+1)
-    c[5] = (b0 >> 1) | (((ctl >> lane) & 1u) << 31);
-    c[6] = b1;
-    c[7] = (b1 >> 1) | ((__funnelshift_rc(ctl, cth, lane + 1) & 1u) << 31);
-    uint32_t all = c[0], any = c[0];
-#pragma unroll
-    for (int k = 1; k < 8; k++) {
-        all &= c[k];
-        any |= c[k];
-    }
-    // cells that are neither all-inside nor all-outside: the only ones with
-    // vertices (every other MC case has at least one triangle)
-    const uint32_t active = (all ^ any) & vmask;
-    const bool has_vertices = __any_sync(0xffffffffu, active != 0u);
-    if (!has_vertices) {
-        if (lane == 0) V.levels[V.level_off[kBlockLevel] + b] = 0u;
-        if (!V.codes_out) return;
-    }
-    // codes of this row (cells outside the grid are masked to 0)
-#pragma unroll
-    for (int k = 0; k < 8; k++) c[k] &= vmask;
-    uint32_t w[8];
-    slices_to_codes(c, w);
-    if (has_vertices) {
-        // the block's vertices: 32 independent count lookups per lane (byte j
-        // of seg = the row's cells 8j .. 8j+7, at most 96), one warp
-        // reduction (inactive cells have codes 0 or 255, count 0)
-        uint32_t seg = 0;
-#pragma unroll
-        for (int i = 0; i < 32; i++) seg += (uint32_t)s_cnt[(w[i >> 2] >> (8 * (i & 3))) & 0xffu] << (8 * (i >> 3));
-        const uint32_t vs = (seg & 0xffu) + ((seg >> 8) & 0xffu) + ((seg >> 16) & 0xffu) + (seg >> 24);
-        const uint32_t total = __reduce_add_sync(0xffffffffu, vs);
-        if (lane == 0) V.levels[V.level_off[kBlockLevel] + b] = total;
-        // codes in Morton order: word q of the slot = quad (qx, qy), cells
-        // (2qx,2qy), (2qx+1,2qy), (2qx,2qy+1), (2qx+1,2qy+1) from rows 2qy
-        // (even lane) and 2qy+1 (odd lane); even lanes store qx 0..7, odd
-        // lanes qx 8..15, each pairing its row with its neighbour's
-        uint32_t p[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) p[i] = __shfl_xor_sync(0xffffffffu, w[i], 1);
-        const bool odd = lane & 1;
-        const uint32_t qy = (uint32_t)lane >> 1;
-        const long long slot = ((long long)z * V.nfy + fy) * V.nfx + fx;
-        uint32_t* dst = V.arena + slot * kSlotWords;
-        // Morton index of quad (qx, qy), qx = (odd ? 8 : 0) + i: the bits of i
-        // (compile-time) and of the lane's part are disjoint
-        const uint32_t qys = (qy & 1u) | ((qy & 2u) << 1) | ((qy & 4u) << 2) | ((qy & 8u) << 3);
-        const uint32_t qbase = (odd ? 0x40u : 0u) | (qys << 1);
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const uint32_t wi = odd ? w[4 + (i >> 1)] : w[i >> 1];  // this lane's word with cells 2qx, 2qx+1
-            const uint32_t pi = odd ? p[4 + (i >> 1)] : p[i >> 1];
-            const uint32_t upper = odd ? wi : pi;  // row 2qy+1
-            const uint32_t lower = odd ? pi : wi;  // row 2qy
-            const uint32_t word = __byte_perm(lower, upper, (i & 1) ? 0x7632 : 0x5410);
-            const uint32_t ispread = (uint32_t)((i & 1) | ((i & 2) << 1) | ((i & 4) << 2));
-            dst[qbase | ispread] = word;
-        }
-        // Morton tile q = lane (cells 32q .. 32q+31, an 8x4 tile at rows
-        // ty .. ty+3, columns tx .. tx+7; Morton bits x0 y0 x1 y1 x2 | y2 x3
-        // y3 x4 y4): its active mask gathered from four rows in Morton order
-        // and its vertices from the rows' segment counts
-        const uint32_t q = (uint32_t)lane;
-        const int ty = 4 * (int)((q & 1u) | ((q >> 1) & 2u) | ((q >> 2) & 4u));
-        const uint32_t tx = 8u * (((q >> 1) & 1u) | ((q >> 2) & 2u));
-        uint32_t r[4], tcnt = 0;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            r[i] = (__shfl_sync(0xffffffffu, active, ty + i) >> tx) & 0xffu;
-            tcnt += (__shfl_sync(0xffffffffu, seg, ty + i) >> tx) & 0xffu;
-        }
-        // rows 0/2 on Morton bit 3 = 0/1 with bit 1 = 0; rows 1/3 shifted by 2 (bit 1 = 1)
-        const uint32_t tmask = spread16(r[0] | (r[2] << 8)) | (spread16(r[1] | (r[3] << 8)) << 2);
-        reinterpret_cast<uint2*>(dst + kSlotTileWord)[lane] = make_uint2(tmask, tcnt);
-    }
-    if (V.codes_out) {
-        const int y = fy * 32 + lane;
-        if (y < V.cells[1]) {
-            uint8_t* row = V.codes_out + ((long long)z * V.cells[1] + y) * V.cells[0] + fx * 32;
-            const int nx = min(32, V.cells[0] - fx * 32);
-#pragma unroll
-            for (int i = 0; i < 32; i++)
-                if (i < nx) row[i] = (uint8_t)(w[i >> 2] >> (8 * (i & 3)));
-        }
-    }
-}
-
-}  // namespace
-
-// Shared memory of a column classifier CTA.  Bit rows are kept for the last
-// kRowBuffers sample layers (indexed by a running layer counter mod
-// kRowBuffers): while a slow warp still classifies the slices of box p
-// (layers 8p-1 .. 8p+7) other warps already convert box p+1 (layers 8p+8 ..
-// 8p+15), so the buffers of the two boxes must not alias.
-constexpr int kRowBuffers = 32;
-
 template <int FT>
 struct ColumnGeom {
     using T = typename std::conditional<FT == kFieldF32, float, uint8_t>::type;
@@ -231,110 +49,32 @@ struct ColumnGeom {
 };
 
 struct ColumnSmem {
-    // 16-byte aligned: warps store 4 rows at a time (uint4), whatever the
-    // number of ring stages before it
-    alignas(16) uint32_t rows[kRowBuffers][36];  // bit x = sample (x0 + x, y0 + r) below iso; [32] = row 32
-    uint64_t col[kRowBuffers];                   // bit r = sample (x0 + 32, y0 + r) below iso; bit 32 = corner
+    ColumnBits bits;
     uint64_t bar[kRingStages];
-    uint8_t cnt[256];
-    // level-5 index of block (0, 0) of slice z, z < kSliceTable: a footprint's
-    // block is that OR its own Morton part (the footprint's bits lie below
-    // the tile's), so a slice costs one load instead of two bit spreads
-    uint32_t zbase[1024];
 };
-constexpr int kSliceTable = 1024;
-static_assert(offsetof(ColumnSmem, rows) % 16 == 0 && (36 * 4) % 16 == 0, "uint4 row stores need 16-byte alignment");
 
-// Bit rows of the nl layers of one box (stage st), layer l stored at
-// running index gl0 + l.  Warp w converts rows 4w .. 4w+3 of every layer;
-// row 32 and column x0+32 of layer g go to warp (g + 3) mod 8.
-static_assert(kWarps == 8 && kLayersPerBox <= kWarps, "a box's layers and slices map onto the 8 warps mod 8");
-static_assert(kRowBuffers % kLayersPerBox == 0, "a box's bit-row buffers never wrap");
-
+// Bit rows of the nl layers of one box (ring stage st).
 template <int FT>
 __device__ __forceinline__ void convert_box(const typename ColumnGeom<FT>::T* st, int nl, uint32_t gl0, float iso,
-                                            int u8_thr, int warp, int lane, ColumnSmem& C) {
+                                            int u8_thr, int warp, int lane, ColumnBits& C) {
     using G = ColumnGeom<FT>;
-    using T = typename G::T;
     // Every sample first, then the ballots and stores: the compiler cannot
     // tell the bit-row stores from the ring stage, so loads issued after a
     // store would wait for it.  A stage always holds kLayersPerBox layers
     // (copies past the volume read zeros), so all of them are read; layers
     // past nl are not stored.
-    T v[kLayersPerBox][4];
-    const T* row = st + 4 * warp * G::BXE + lane;
+    BoxSamples<typename G::T> s;
+    const typename G::T* row = st + 4 * warp * G::BXE + lane;
 #pragma unroll
     for (int l = 0; l < kLayersPerBox; l++)
 #pragma unroll
-        for (int i = 0; i < 4; i++) v[l][i] = row[l * G::LAYER + i * G::BXE];
-    const int le = (int)(((uint32_t)warp - gl0 - 3u) & 7u);  // the layer whose row 32 and column 32 this warp takes
-    const T* layer = st + (le < kLayersPerBox ? le : 0) * G::LAYER;  // inside the stage for any box depth
-    const T e_row = layer[32 * G::BXE + lane], e_col = layer[lane * G::BXE + 32], e_corner = layer[32 * G::BXE + 32];
-    // gl0 is a multiple of kLayersPerBox and kRowBuffers of that, so a box's
-    // buffers are g0 .. g0 + kLayersPerBox - 1 without wrapping
-    const uint32_t g0 = gl0 & (kRowBuffers - 1);
-    uint4* const rows_w = reinterpret_cast<uint4*>(&C.rows[g0][4 * warp]);
-#pragma unroll
-    for (int l = 0; l < kLayersPerBox; l++) {
-        const uint32_t b0 = __ballot_sync(0xffffffffu, below<FT>(v[l][0], iso, u8_thr));
-        const uint32_t b1 = __ballot_sync(0xffffffffu, below<FT>(v[l][1], iso, u8_thr));
-        const uint32_t b2 = __ballot_sync(0xffffffffu, below<FT>(v[l][2], iso, u8_thr));
-        const uint32_t b3 = __ballot_sync(0xffffffffu, below<FT>(v[l][3], iso, u8_thr));
-        if (l < nl && lane == 0) rows_w[l * (36 / 4)] = make_uint4(b0, b1, b2, b3);
-    }
-    const uint32_t r32 = __ballot_sync(0xffffffffu, below<FT>(e_row, iso, u8_thr));
-    const uint32_t col = __ballot_sync(0xffffffffu, below<FT>(e_col, iso, u8_thr));
-    const bool corner = below<FT>(e_corner, iso, u8_thr);
-    if (le < nl && lane == 0) {
-        const uint32_t buf = g0 + (uint32_t)le;
-        C.rows[buf][32] = r32;
-        C.col[buf] = (uint64_t)col | ((uint64_t)corner << 32);
-    }
-}
-
-// Morton part of footprint (fx, fy) in a block index.
-__device__ __forceinline__ uint32_t footprint_morton(int fx, int fy) {
-    return morton_spread16((uint32_t)fx) | (morton_spread16((uint32_t)fy) << 1);
-}
-
-// The slice table for slices 0 .. min(cells, kSliceTable)-1 (all threads).
-__device__ __forceinline__ void fill_slice_table(const Volume& V, ColumnSmem& C) {
-    const int n = min(V.cells[2], kSliceTable);
-    for (int z = threadIdx.x; z < n; z += blockDim.x) C.zbase[z] = (uint32_t)column_block_index(V, z, 0, 0);
-}
-
-__device__ __forceinline__ uint32_t slice_block(const Volume& V, const ColumnSmem& C, int z, uint32_t fm) {
-    return (z < kSliceTable ? C.zbase[z] : (uint32_t)column_block_index(V, z, 0, 0)) | fm;
-}
-
-// After the box barrier: the slices whose upper layer arrived in this box
-// (column-relative slices lb-1 .. lb+nl-2), warp (glu + slice) mod 8 each, so
-// the work rotates over the warps from box to box.  glu = running index of
-// the column's layer 0.
-__device__ __forceinline__ void classify_box_slices(const Volume& V, int z0, int fx, int fy, uint32_t fm, int lb,
-                                                    int nl, uint32_t glu, int warp, int lane, uint32_t vmask,
-                                                    bool full, ColumnSmem& C) {
-    // the slice of this warp, if any.  glu + lb is the running index of the
-    // box's first layer, a multiple of kLayersPerBox: with 8-layer boxes the
-    // warp's offset in the box is the same in every box
-    const uint32_t w1 = kLayersPerBox == 8 ? (uint32_t)(warp + 1) & 7u
-                                           : ((uint32_t)warp - (glu + (uint32_t)lb - 1u)) & 7u;
-    const int sl = lb - 1 + (int)w1;
-    if (sl >= 0 && sl <= lb + nl - 2) {
-        const uint32_t g = glu + (uint32_t)sl;
-        const uint32_t bb = g & (kRowBuffers - 1), bt = (g + 1u) & (kRowBuffers - 1);
-        const int z = z0 + sl;
-        classify_slice_warp(V, z, fx, fy, slice_block(V, C, z, fm), lane, vmask, full, C.rows[bb], C.col[bb],
-                            C.rows[bt], C.col[bt], C.cnt);
-    }
-}
-
-// Cells of row `lane` of footprint (x0, y0) inside the grid (masked codes are
-// 0, shadergen.cpp:112-125).
-__device__ __forceinline__ uint32_t row_mask(const Volume& V, int x0, int y0, int lane) {
-    const int xv = V.cells[0] - x0;
-    const uint32_t xmask = xv >= 32 ? 0xffffffffu : ((1u << xv) - 1u);
-    return (y0 + lane < V.cells[1]) ? xmask : 0u;
+        for (int i = 0; i < 4; i++) s.v[l][i] = row[l * G::LAYER + i * G::BXE];
+    const int le = edge_layer(gl0, warp);
+    const typename G::T* layer = st + (le < kLayersPerBox ? le : 0) * G::LAYER;  // inside the stage for any box depth
+    s.row = layer[32 * G::BXE + lane];
+    s.col = layer[lane * G::BXE + 32];
+    s.corner = layer[32 * G::BXE + 32];
+    box_bits(s, nl, gl0, iso, u8_thr, warp, lane, C);
 }
 
 template <int FT>
@@ -363,8 +103,7 @@ __device__ __forceinline__ void classify_column_body(const CUtensorMap* tmap, co
     const float iso = V.binary ? 0.5f : V.iso;
     const int u8_thr = V.u8_thr;
 
-    C.cnt[tid] = c_vertex_count[tid];
-    fill_slice_table(V, C);
+    fill_column_tables(V, C.bits, z0, z1);
     const uint32_t fm = footprint_morton(fx, fy);
     if (tid == 0) {
         for (int s = 0; s < kRingStages; s++) mbar_init(&C.bar[s], 1);
@@ -395,7 +134,7 @@ __device__ __forceinline__ void classify_column_body(const CUtensorMap* tmap, co
         if (!mbar_wait_bounded(&C.bar[s], parity, V.wait_limit_ns, &V.ctrl->status, kStatusTimeout)) timed_out = true;
         if (!timed_out)
             convert_box<FT>(reinterpret_cast<const typename G::T*>(s_ring + s * G::STAGE_STRIDE), nl, (uint32_t)lb,
-                            iso, u8_thr, warp, lane, C);
+                            iso, u8_thr, warp, lane, C.bits);
         // the only CTA barrier of a box: stage s consumed, bit rows of layers
         // lb .. lb+nl-1 ready, and a uniform decision on a timed-out wait
         if (__syncthreads_or(timed_out)) break;
@@ -404,7 +143,7 @@ __device__ __forceinline__ void classify_column_body(const CUtensorMap* tmap, co
             tma_load_3d(s_ring + s * G::STAGE_STRIDE, tmap, x0, y0, z0 + (k + kRingStages) * kLayersPerBox,
                         &C.bar[s], pol);
         }
-        classify_box_slices(V, z0, fx, fy, fm, lb, nl, 0u, warp, lane, vmask, full, C);
+        classify_box_slices(V, z0, fx, fy, fm, lb, nl, 0u, warp, lane, vmask, full, C.bits);
     }
     if (timed_out) {
         // drain the boxes still in flight (bounded) before the CTA exits
@@ -454,8 +193,7 @@ __global__ void __launch_bounds__(kThreads) classify_columns(const __grid_consta
     };
 
     __shared__ int s_early;
-    C.cnt[tid] = c_vertex_count[tid];
-    fill_slice_table(V, C);
+    fill_column_tables(V, C.bits, 0, V.cells[2]);
     if (tid == 0) {
         for (int s = 0; s < kRingStages; s++) mbar_init(&C.bar[s], 1);
         mbar_fence_init();
@@ -532,7 +270,7 @@ __global__ void __launch_bounds__(kThreads) classify_columns(const __grid_consta
         const int nl = min(kLayersPerBox, nlayers - lb);
         if (ok && tag.x >= 0)
             convert_box<FT>(reinterpret_cast<const typename G::T*>(s_ring + s * G::STAGE_STRIDE), nl,
-                            pos * kLayersPerBox, iso, u8_thr, warp, lane, C);
+                            pos * kLayersPerBox, iso, u8_thr, warp, lane, C.bits);
         // the only CTA barrier of a box (uniform decision on a timed-out wait);
         // the producer rewrites the stage and its tag only after it
         if (__syncthreads_or(!ok)) {
@@ -544,7 +282,7 @@ __global__ void __launch_bounds__(kThreads) classify_columns(const __grid_consta
         const uint32_t vmask = (uint32_t)lane < (rm.y & 0xffu) ? rm.x : 0u;  // == row_mask(V, 32 fx, 32 fy, lane)
         const bool full = (rm.y >> 31) != 0u;
         classify_box_slices(V, z0, fx, fy, fm, lb, nl, (pos - (uint32_t)k) * kLayersPerBox, warp, lane, vmask, full,
-                            C);
+                            C.bits);
     }
     if (timed_out && tid == 0) {
         // drain the boxes still in flight (bounded) before the CTA exits
@@ -829,8 +567,7 @@ static int column_ctas_per_sm() {
 
 cudaError_t launch_classify(const Volume& V, const CUtensorMap* tmap, int max_ctas, cudaStream_t st) {
     if (V.column_layout && tmap) {
-        const int nz = (V.cells[2] + V.column_slices - 1) / V.column_slices;
-        const int ncolumns = V.nfx * V.nfy * nz;
+        const int ncolumns = column_count(V);
         // persistent: every resident CTA slot (max_ctas = 16 per SM)
         const int slots = (max_ctas / 16) * column_ctas_per_sm();
         const int grid = ncolumns < slots ? ncolumns : slots;
@@ -841,6 +578,15 @@ cudaError_t launch_classify(const Volume& V, const CUtensorMap* tmap, int max_ct
         else
             return launch_dependent(classify_columns<kFieldUNorm8>, grid, kThreads, kRingBytesU8, st, *tmap, V,
                                     ncolumns);
+    } else if (V.column_layout) {
+        const int grid = column_count(V);
+        switch (V.ftype) {
+            case kFieldF32: return launch_dependent(classify_columns_direct<kFieldF32>, grid, kThreads, 0, st, V);
+            case kFieldU8: return launch_dependent(classify_columns_direct<kFieldU8>, grid, kThreads, 0, st, V);
+            case kFieldUNorm8: return launch_dependent(classify_columns_direct<kFieldUNorm8>, grid, kThreads, 0, st, V);
+            case kFieldF32X4: return launch_dependent(classify_columns_direct<kFieldF32X4>, grid, kThreads, 0, st, V);
+            default: return launch_dependent(classify_columns_direct<kFieldFunctor>, grid, kThreads, 0, st, V);
+        }
     } else {
         const long long nb = V.nblocks;
         const int grid = (int)(nb < (long long)max_ctas ? nb : (long long)max_ctas);

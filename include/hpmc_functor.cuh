@@ -7,7 +7,7 @@
  * normals -- that the application writes, and compiles it into the
  * HistoPyramid's shaders.  Here the application writes the same function as a
  * CUDA functor type and compiles it in its own .cu file with this header:
- * HPMC_FIELD_FUNCTOR instantiates the library's generic classifier and its
+ * HPMC_FIELD_FUNCTOR instantiates the library's direct classifiers and its
  * traversal for that type in the application's own device code and defines
  * the launch table that HPMCregisterFieldFunctor takes.  After registration,
  * HPMCsetFieldCustom(h, name, unit, gradient) selects the functor by name, and
@@ -37,8 +37,7 @@
  * the values at the edge ends and n = iso - lerp(grad a, grad b, t), as the
  * reference does (shadergen.cpp:539-551), or -lerp(...) with
  * HPMC_NORMALS_CENTRAL; without gradient mode the normals are differences of
- * value() like the reference's.  Functor fields take the generic (per-block)
- * classifier.  Adjoint and indexed extraction are not available for them.
+ * value() like the reference's.  Adjoint and indexed extraction are not available for them.
  *
  * Build the .cu with nvcc -gencode arch=compute_100a,code=sm_100a -std=c++17
  * and the include paths of include/ and hpmc_b200/csrc/ (the kernel bodies and
@@ -51,6 +50,7 @@
 
 #include "hpmc.h"
 #include "hpmc_classify_core.cuh"
+#include "hpmc_column_core.cuh"
 #include "hpmc_traverse_core.cuh"
 
 namespace hpmc {
@@ -60,6 +60,9 @@ namespace hpmc {
 template <class F>
 int user_classify(const void* volume, int grid, void* stream) {
     const Volume& V = *static_cast<const Volume*>(volume);
+    if (V.column_layout)
+        return launch_dependent(classify_columns_direct<kFieldUser, F>, column_count(V), kThreads, 0,
+                                static_cast<cudaStream_t>(stream), V) == cudaSuccess ? HPMC_OK : HPMC_ERR_CUDA;
     classify_blocks<kFieldUser, F><<<grid, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(V);
     return cudaGetLastError() == cudaSuccess ? HPMC_OK : HPMC_ERR_CUDA;
 }

@@ -1,0 +1,36 @@
+"""The direct column classifier (column layouts without a tensor map) at the
+edges of its tiles: footprints of 17, 32, 33 and 64 cells with remainders,
+columns of one slice, of a whole box of 8 layers and one layer more.  Codes,
+levels, order and geometry against the oracle (bit-exact topology, the parity
+tolerances of tests/gpu_helpers.py)."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from tests.gpu_helpers import compare, oracle_expect, run_gpu
+
+pytestmark = pytest.mark.gpu
+
+# (z, y, x)
+SHAPES = [(2, 18, 18), (8, 33, 33), (9, 34, 18), (10, 18, 65), (17, 66, 33), (65, 35, 34)]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("kind", ["f32", "f32_pitched", "u8", "unorm8", "f32x4", "functor"])
+def test_direct_columns(hpmc, oracle, shape, kind):
+    rng = np.random.default_rng(sum(shape) + len(kind))
+    kw, iso, okw = {}, 0.0, {}
+    if kind.startswith("f32"):
+        field = rng.normal(size=shape + ((4,) if kind == "f32x4" else ())).astype(np.float32)
+        kw = {"pitch_pad": 3} if kind == "f32_pitched" else {"texture": True} if kind == "f32x4" else {}
+    elif kind == "functor":
+        field, iso = oracle.Functor("hpmc:cayley", [], shape), 0.1
+    else:
+        field = rng.integers(100, 156, size=shape).astype(np.uint8)
+        okw = {"unorm": kind == "unorm8"}
+        iso = 128.0 / 255.0 if kind == "unorm8" else 128.0
+    g = run_gpu(hpmc, field, iso, **kw, **okw)
+    row_bytes = {"f32": 4 * shape[2], "f32_pitched": 4 * (shape[2] + 3), "u8": shape[2], "unorm8": shape[2]}.get(kind, 1)
+    assert g["path"] == (1 if row_bytes % 16 == 0 else 0)  # a tensor map covers rows of 16-byte multiples
+    compare(g, oracle_expect(oracle, field, iso, **okw))
