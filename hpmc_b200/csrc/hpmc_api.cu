@@ -84,8 +84,8 @@ struct HPMCHistoPyramid {
     // reads the other set (Volume::overlap).  One control block.
     uint32_t* d_levels = nullptr;  // nsets x levels_cap entries
     size_t levels_cap = 0;         // entries per set
-    uint32_t* d_arena = nullptr;   // nsets x arena_cap slots
-    size_t arena_cap = 0;          // slots per set
+    uint32_t* d_arena = nullptr;   // nsets x arena_cap words
+    size_t arena_cap = 0;          // words per set
     int nsets = 0;
     int set = 0;                   // the set of the last build
     Ctrl* d_ctrl = nullptr;
@@ -203,8 +203,9 @@ bool setup(HPMCHistoPyramid* h) {
     hpmc::host::volume_layout(V, h->lattice, h->cells, h->extent, L, &levels_total, &slots);
     V.column_slices = hpmc::host::default_column_slices(V, h->constants->num_sms);
     const int nsets = V.column_layout ? 2 : 1;
+    const size_t arena_words = (size_t)slots * V.slot_words;
     // (re)allocate
-    if ((size_t)levels_total > h->levels_cap || (size_t)slots > h->arena_cap || nsets > h->nsets || !h->d_ctrl) {
+    if ((size_t)levels_total > h->levels_cap || arena_words > h->arena_cap || nsets > h->nsets || !h->d_ctrl) {
         if (h->d_ctrl && cudaStreamSynchronize(h->stream) != cudaSuccess) {
             cudaGetLastError();
             h->status = HPMC_ERR_CUDA;
@@ -212,7 +213,7 @@ bool setup(HPMCHistoPyramid* h) {
         }
         release_device(h);
         if (cudaMalloc(&h->d_levels, sizeof(uint32_t) * levels_total * nsets) != cudaSuccess ||
-            cudaMalloc(&h->d_arena, hpmc::kSlotBytes * (size_t)slots * nsets) != cudaSuccess ||
+            cudaMalloc(&h->d_arena, sizeof(uint32_t) * arena_words * nsets) != cudaSuccess ||
             cudaMalloc(&h->d_ctrl, sizeof(Ctrl)) != cudaSuccess) {
             cudaGetLastError();
             release_device(h);
@@ -220,7 +221,7 @@ bool setup(HPMCHistoPyramid* h) {
             return false;
         }
         h->levels_cap = (size_t)levels_total;
-        h->arena_cap = (size_t)slots;
+        h->arena_cap = arena_words;
         h->nsets = nsets;
     }
     // every set's levels start at zero (padding blocks' level-5 entries stay zero)
@@ -245,7 +246,7 @@ int traverse_grid(const HPMCHistoPyramid* h) {
     const HPMCConstants* c = h->constants;
     int grid = c->num_sms * c->traverse_ctas_per_sm;
     if (h->count_valid) {
-        const unsigned long long per_cta = 32ull * hpmc::kTraverseRounds * hpmc::kWarps;
+        const unsigned long long per_cta = 32ull * hpmc::kMinRounds * hpmc::kWarps;
         const unsigned long long need = (h->count_cached + per_cta - 1) / per_cta;
         grid = (int)std::max<unsigned long long>(1, std::min<unsigned long long>((unsigned long long)grid, need));
     }
@@ -487,7 +488,7 @@ void HPMCbuildHistopyramid(HPMCHistoPyramid* h, GLfloat threshold) {
     if (V.column_layout && h->nsets == 2) {
         h->set ^= 1;
         V.levels = h->d_levels + (size_t)h->set * h->levels_cap;
-        V.arena = h->d_arena + (size_t)h->set * h->arena_cap * hpmc::kSlotWords;
+        V.arena = h->d_arena + (size_t)h->set * h->arena_cap;
     }
     V.overlap = may_overlap_extraction(h) ? 1 : 0;
     h->threshold = threshold;
@@ -896,6 +897,10 @@ namespace {
 static __device__ __align__(256) unsigned char g_static_scratch[HPMC_STATIC_SCRATCH_BYTES];
 
 constexpr int kStaticMaxDevices = 64;
+constexpr size_t kStaticBlockBytes = 1280;  // scratch reserved per block (a slot takes at most this)
+static_assert(sizeof(uint32_t) * hpmc::kCodeSlotWords <= kStaticBlockBytes &&
+                  sizeof(uint32_t) * hpmc::kRowSlotWords <= kStaticBlockBytes,
+              "a block's slot fits its share of the scratch");
 
 struct StaticDeviceState {
     unsigned char* scratch = nullptr;  // device address of g_static_scratch on this device
@@ -971,7 +976,8 @@ extern "C" int HPMCextractStatic(const void* field, int scalar_type, GLsizei x_s
     // carve the scratch: control block | dense levels | block codes
     const size_t ctrl_bytes = align256(sizeof(Ctrl));
     const size_t levels_bytes = align256(sizeof(uint32_t) * (size_t)level_entries_total);
-    const size_t arena_bytes = hpmc::kSlotBytes * (size_t)slots;
+    // the volumes the scratch takes are those for which 1,280 bytes a block fit
+    const size_t arena_bytes = kStaticBlockBytes * (size_t)slots;
     if (ctrl_bytes + levels_bytes + arena_bytes > (size_t)HPMC_STATIC_SCRATCH_BYTES) return HPMC_ERR_TOO_LARGE;
     unsigned char* base = dev->scratch;
     V.ctrl = reinterpret_cast<Ctrl*>(base);

@@ -7,7 +7,7 @@
 // Device memory of a batch (one allocation):
 //   batch control block | per-volume control blocks | descriptors |
 //   tensor maps | brick, reduce-chunk and work-item prefix arrays |
-//   output offsets | dense levels of every volume | block-code arenas
+//   output offsets | dense levels of every volume | block arenas
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -309,8 +309,9 @@ int HPMCcreateBatch(HPMCConstants* c, const HPMCBatchVolume* volumes, int count,
             b->column[v] = hpmc::host::encode_column_map(&b->tmaps[v], s.field, stype, lattice, rp, sp) ? 1 : 0;
         lev_off[v] = lev_total;
         lev_total += lev;  // a multiple of 4 entries: every volume's levels stay 16-byte aligned
+        V.arena_slots = slots;
         arena_off[v] = arena_total;
-        arena_total += slots;
+        arena_total += slots * V.slot_words;
         b->reduce_start[v] = chunks;
         const long long n5 = hpmc::level_entries(V.size_l2, hpmc::kBlockLevel);
         chunks += (uint32_t)std::max(1ll, (n5 + 1023) / 1024);
@@ -340,7 +341,7 @@ int HPMCcreateBatch(HPMCConstants* c, const HPMCBatchVolume* volumes, int count,
     const size_t o_vbase = off;
     off = align_up(off + sizeof(unsigned long long) * (count + 1), 256);
     const size_t o_arena = off;
-    off += hpmc::kSlotBytes * (size_t)arena_total;
+    off += sizeof(uint32_t) * (size_t)arena_total;
     if (cudaMalloc(&b->d_base, off) != cudaSuccess) {
         cudaGetLastError();
         delete b;
@@ -366,8 +367,7 @@ int HPMCcreateBatch(HPMCConstants* c, const HPMCBatchVolume* volumes, int count,
     for (int v = 0; v < count; v++) {
         Volume& V = b->hv[v];
         V.levels = d_levels + lev_off[v];
-        V.arena = d_arena + (size_t)hpmc::kSlotWords * (size_t)arena_off[v];
-        V.arena_slots = (v + 1 < count ? arena_off[v + 1] : arena_total) - arena_off[v];
+        V.arena = d_arena + arena_off[v];
         V.ctrl = b->d_ctrls + v;
     }
     apply_column_slices(b);

@@ -25,13 +25,13 @@ __device__ __forceinline__ int find_segment(const uint32_t* start, int n, uint32
     return lo;
 }
 
-// Copy of a volume descriptor into shared memory by `nthreads` threads
-// numbered `t` (a CTA or a warp).
+// Copy of a volume descriptor (without its functor: batches take array fields)
+// into shared memory by `nthreads` threads numbered `t` (a CTA or a warp).
 __device__ __forceinline__ void copy_volume(Volume* dst, const Volume* src, int t, int nthreads) {
     static_assert(sizeof(Volume) % 8 == 0, "Volume is copied in 8-byte words");
     const uint2* s = reinterpret_cast<const uint2*>(src);
     uint2* d = reinterpret_cast<uint2*>(dst);
-    for (int i = t; i < (int)(sizeof(Volume) / 8); i += nthreads) d[i] = __ldg(s + i);
+    for (int i = t; i < (int)(kVolumeHead / 8); i += nthreads) d[i] = __ldg(s + i);
 }
 
 }  // namespace hpmc

@@ -53,9 +53,9 @@ __device__ __forceinline__ void write_codes(const Volume& V, uint32_t packed, in
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// Generic classification: CTA = one 32x32 block of the virtual cell grid,
-// for any tiling (tiles narrower than 32 cells), unaligned pitches and
-// functor fields.  Each thread loads its quad's 3x3x2 samples directly; the
+// Generic classification: CTA = one 32x32 block of the virtual cell grid, for
+// layouts whose tiles are narrower than 32 cells (a block then holds cells of
+// several slices), whatever the pitch or the field source.  Each thread loads its quad's 3x3x2 samples directly; the
 // quads are numbered in Morton order, so thread t's four codes are word t of
 // the block's arena slot, and threads 8l .. 8l+7 (one eighth of a warp) hold
 // Morton tile l, whose active mask and vertices they combine by shuffles.
@@ -116,9 +116,12 @@ __device__ __forceinline__ void classify_block_body(const Volume& V, uint64_t b,
     for (int w = 0; w < kWarps; w++) total += s_warp[w];
     if (tid == 0) V.levels[V.level_off[kBlockLevel] + b] = total;
     if (total) {
-        uint32_t* slot = V.arena + block_slot(V, b) * kSlotWords;
+        uint32_t* slot = V.arena + block_slot(V, b) * kCodeSlotWords;
         slot[tid] = packed;
-        if ((tid & 7) == 0) reinterpret_cast<uint2*>(slot + kSlotTileWord)[tid >> 3] = make_uint2(tmask, tcnt);
+        if ((tid & 7) == 0) {
+            slot[kCodeSlotMasks + (tid >> 3)] = tmask;
+            reinterpret_cast<uint16_t*>(slot + kCodeSlotCounts)[tid >> 3] = (uint16_t)tcnt;
+        }
     }
     __syncthreads();
 }

@@ -59,17 +59,10 @@ __device__ __forceinline__ void slices_to_codes(const uint32_t c[8], uint32_t w[
     }
 }
 
-// 16 bits -> Morton positions of an 8x2 cell tile: bit x of the low byte goes
-// to bit (x0 | x1 << 2 | x2 << 4), bit x of the high byte to that + 8.
-__device__ __forceinline__ uint32_t spread16(uint32_t t) {
-    t = (t | (t << 12)) & 0x0F0F0F0Fu;
-    return (t | (t << 2)) & 0x33333333u;
-}
-
 // One warp: classify slice z of footprint (fx, fy) from sample-bit rows of the
 // lower layer (rows_b/col_b) and the upper layer (rows_t/col_t).  Every block
-// gets its level-5 count; blocks with vertices store their codes in Morton
-// order in their slot.  full: every cell of the footprint lies inside the
+// gets its level-5 count; blocks with vertices store their sample bits and
+// their tiles' vertices in their slot.  full: every cell of the footprint lies inside the
 // grid (vmask is all ones in every lane).  b: the block's level-5 index,
 // column_block_index(V, z, fx, fy).
 __device__ __forceinline__ void classify_slice_warp(const Volume& V, int z, int fx, int fy, uint32_t b, int lane,
@@ -134,47 +127,21 @@ __device__ __forceinline__ void classify_slice_warp(const Volume& V, int z, int 
         const uint32_t vs = (seg & 0xffu) + ((seg >> 8) & 0xffu) + ((seg >> 16) & 0xffu) + (seg >> 24);
         const uint32_t total = __reduce_add_sync(0xffffffffu, vs);
         if (lane == 0) V.levels[V.level_off[kBlockLevel] + b] = total;
-        // codes in Morton order: word q of the slot = quad (qx, qy), cells
-        // (2qx,2qy), (2qx+1,2qy), (2qx,2qy+1), (2qx+1,2qy+1) from rows 2qy
-        // (even lane) and 2qy+1 (odd lane); even lanes store qx 0..7, odd
-        // lanes qx 8..15, each pairing its row with its neighbour's
-        uint32_t p[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) p[i] = __shfl_xor_sync(0xffffffffu, w[i], 1);
-        const bool odd = lane & 1;
-        const uint32_t qy = (uint32_t)lane >> 1;
-        const long long slot = ((long long)z * V.nfy + fy) * V.nfx + fx;
-        uint32_t* dst = V.arena + slot * kSlotWords;
-        // Morton index of quad (qx, qy), qx = (odd ? 8 : 0) + i: the bits of i
-        // (compile-time) and of the lane's part are disjoint
-        const uint32_t qys = (qy & 1u) | ((qy & 2u) << 1) | ((qy & 4u) << 2) | ((qy & 8u) << 3);
-        const uint32_t qbase = (odd ? 0x40u : 0u) | (qys << 1);
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const uint32_t wi = odd ? w[4 + (i >> 1)] : w[i >> 1];  // this lane's word with cells 2qx, 2qx+1
-            const uint32_t pi = odd ? p[4 + (i >> 1)] : p[i >> 1];
-            const uint32_t upper = odd ? wi : pi;  // row 2qy+1
-            const uint32_t lower = odd ? pi : wi;  // row 2qy
-            const uint32_t word = __byte_perm(lower, upper, (i & 1) ? 0x7632 : 0x5410);
-            const uint32_t ispread = (uint32_t)((i & 1) | ((i & 2) << 1) | ((i & 4) << 2));
-            dst[qbase | ispread] = word;
-        }
-        // Morton tile q = lane (cells 32q .. 32q+31, an 8x4 tile at rows
-        // ty .. ty+3, columns tx .. tx+7; Morton bits x0 y0 x1 y1 x2 | y2 x3
-        // y3 x4 y4): its active mask gathered from four rows in Morton order
-        // and its vertices from the rows' segment counts
+        // the block's sample bits (see kRowSlotWords)
+        uint32_t* dst = V.arena + (((long long)z * V.nfy + fy) * V.nfx + fx) * kRowSlotWords;
+        dst[lane] = a0;
+        dst[32 + lane] = b0;
+        if (lane == 0) *reinterpret_cast<uint4*>(dst + 64) = make_uint4(rows_b[32], rows_t[32], cbl, ctl);
+        if (lane == 1) dst[68] = (cbh & 1u) | ((cth & 1u) << 1);
+        // Morton tile `lane` is the 8x4 cells at rows ty .. ty+3, columns tx ..
+        // tx+7: its vertices from the rows' segment counts
         const uint32_t q = (uint32_t)lane;
-        const int ty = 4 * (int)((q & 1u) | ((q >> 1) & 2u) | ((q >> 2) & 4u));
-        const uint32_t tx = 8u * (((q >> 1) & 1u) | ((q >> 2) & 2u));
-        uint32_t r[4], tcnt = 0;
+        const int ty = morton_tile_y(q);
+        const uint32_t tx = morton_tile_x(q);
+        uint32_t tcnt = 0;
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            r[i] = (__shfl_sync(0xffffffffu, active, ty + i) >> tx) & 0xffu;
-            tcnt += (__shfl_sync(0xffffffffu, seg, ty + i) >> tx) & 0xffu;
-        }
-        // rows 0/2 on Morton bit 3 = 0/1 with bit 1 = 0; rows 1/3 shifted by 2 (bit 1 = 1)
-        const uint32_t tmask = spread16(r[0] | (r[2] << 8)) | (spread16(r[1] | (r[3] << 8)) << 2);
-        reinterpret_cast<uint2*>(dst + kSlotTileWord)[lane] = make_uint2(tmask, tcnt);
+        for (int i = 0; i < 4; i++) tcnt += (__shfl_sync(0xffffffffu, seg, ty + i) >> tx) & 0xffu;
+        reinterpret_cast<uint16_t*>(dst + kRowSlotCounts)[lane] = (uint16_t)tcnt;
     }
     if (V.codes_out) {
         const int y = fy * 32 + lane;

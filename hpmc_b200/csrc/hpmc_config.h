@@ -23,8 +23,12 @@ constexpr int kColumnSliceChoices[4] = {63, 31, 15, 7};
 constexpr int kColumnsPerSm = 24;
 
 // Traversal: top pyramid entries cached in shared memory per CTA
-// (levels with <= 1024 entries: 1 + 4 + ... + 1024, each padded to 4).
-constexpr int kTopCacheEntries = 1368;
+// (levels with <= 256 entries: 1 + 4 + ... + 256, each padded to 4).
+constexpr int kTopCacheEntries = 344;
+// Resident extraction CTAs per SM (registers; see the note at the kernel).
+constexpr int kTraverseCtas = 3;
+// Rounds of 32 vertices a warp of the single-volume traversal takes at least.
+constexpr int kMinRounds = 4;
 // Vertices per warp work item (R rounds of 32) of the batched traversal (its
 // default; the autotuner chooses) and of the host's grid sizing; the
 // single-volume traversal gives each warp one contiguous range instead.

@@ -15,15 +15,16 @@
 //     count as uint32 -- level j equals the reference's mip level j flattened
 //     channel by channel (level j texel t, channel c <-> entry 4*morton(t)+c);
 //   * below block level nothing is stored densely: each block with a non-zero
-//     count gets an "arena" slot holding its 1024 MC codes in Morton order.
-//     A traversal warp that enters the block turns them into the block's
-//     active-cell list in its own shared memory -- the cells with vertices,
-//     in Morton (= vertex) order, each with its MC code and the
-//     block-relative index of its first vertex.  Levels 0..4 of the reference
-//     are thus implied by the codes: the count of a Morton range of cells is
-//     the difference of two list starts.  Cells of empty blocks are all
-//     inside or all outside and are not needed.
+//     count gets an "arena" slot.  Column layout (every block inside one slice
+//     tile): the block's 33x33 sample bits (below the iso-value or not) of its
+//     lower and upper layer, 288 bytes, from which a traversal warp derives
+//     active cells, MC codes and crossed edges.  Otherwise: the block's 1024 MC
+//     codes in Morton order and the active mask of each of its 32-cell Morton
+//     tiles.  Levels 0..4 of the reference are thus implied: the traversal warp
+//     counts the vertices of the active cells in Morton (= vertex) order.
+//     Cells of empty blocks are all inside or all outside and are not needed.
 #pragma once
+#include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -35,26 +36,20 @@ constexpr int kBlockLevel = 5;       // 4^5 keys per block
 constexpr int kBlockKeys = 1024;
 constexpr int kMaxLevels = 40;
 
-// Arena slot of a non-empty block: its codes in Morton order, four per word
-// (cell 4i + c in byte c of word i), then per Morton tile t of 32 cells
-// (t = 0..31) the pair {active-cell mask (bit i = cell 32t + i), vertices} at
-// words kSlotTileWord + 2t, +1.
-constexpr int kSlotTileWord = kBlockKeys / 4;
-constexpr int kSlotWords = kSlotTileWord + 64;
-constexpr size_t kSlotBytes = sizeof(uint32_t) * (size_t)kSlotWords;
-
-// Active-cell list of one block (a traversal warp's shared memory): one word
-// per cell with vertices, in Morton order,
-//     start << 18 | code << 10 | cell
-// start = block-relative index of the cell's first vertex (< 15 * 1024),
-// code = MC case, cell = Morton index of the cell in the block.  The last
-// entry is followed by kListSentinels words of all ones (start 16383, past
-// any vertex), so a warp may read the 32 entries after any list position
-// without knowing the list's length.
-constexpr int kListSentinels = 32;
-constexpr int kListWords = kBlockKeys + kListSentinels;
-constexpr uint32_t kListSentinel = 0xffffffffu;
-constexpr int kListStartShift = 18;
+// Arena slot of a non-empty block, column layout: bit x of word y (32 + y) =
+// sample (x, y) of the lower (upper) layer below the iso-value, y = 0..31;
+// words 64, 65 = row 32 of the lower and the upper layer; bit y of words 66,
+// 67 = sample (32, y); bits 0 and 1 of word 68 = sample (32, 32).  Samples past
+// the lattice are unspecified: the traversal masks cells outside the grid.
+// Then, at word kRowSlotCounts, the vertices of each 32-cell Morton tile
+// (cells 32t .. 32t + 31, t = 0..31), uint16 each.
+constexpr int kRowSlotCounts = 72;
+constexpr int kRowSlotWords = kRowSlotCounts + 16;
+// Otherwise: the codes in Morton order, four per word (cell 4i + c in byte c
+// of word i), then the tiles' active masks and, uint16 each, their vertices.
+constexpr int kCodeSlotMasks = kBlockKeys / 4;
+constexpr int kCodeSlotCounts = kCodeSlotMasks + 32;
+constexpr int kCodeSlotWords = kCodeSlotCounts + 16;
 
 enum FieldType : int {
     kFieldF32 = 0,      // float
@@ -136,13 +131,12 @@ struct Volume {
     int column_layout;
     int nfx, nfy;                      // 32-cell footprints per slice in x, y
     int column_slices;                 // slices per column CTA
-    uint32_t* arena;                   // kSlotWords words (one block's codes) per slot
+    uint32_t* arena;                   // slot_words words per slot
+    int slot_words;                    // kRowSlotWords (column layout) or kCodeSlotWords
     long long arena_slots;             // capacity of the arena
     Ctrl* ctrl;
     // optional capture of every cell's code, [cz][cy][cx] (inspection)
     uint8_t* codes_out;
-    // custom field
-    FunctorParams functor;
     unsigned long long vertex_base;    // first output index of this volume (batched)
     // bounded waits of the column classifier (kWaitLimitNs unless a test lowers it)
     unsigned long long wait_limit_ns;
@@ -157,7 +151,11 @@ struct Volume {
     // (two alternating sets) and the field is none of that extraction's
     // outputs.  0: every CTA waits for the previous grid first.
     int overlap;
+    // custom field; the last member, so that kernels of array fields can keep
+    // copies of the members before it only (kVolumeHead bytes)
+    FunctorParams functor;
 };
+constexpr size_t kVolumeHead = offsetof(Volume, functor) / 8 * 8 + 8;
 
 // --- Morton helpers (X on even bits) ---------------------------------------
 __host__ __device__ __forceinline__ uint32_t morton_compact(uint64_t v) {
@@ -185,6 +183,20 @@ __host__ __device__ __forceinline__ void morton10(uint32_t m, int& cx, int& cy) 
     y = (y | (y >> 1)) & 0x133u; y = (y | (y >> 2)) & 0x10fu; y = (y | (y >> 4)) & 0x1fu;
     cx = (int)x;
     cy = (int)y;
+}
+
+// First column and row of Morton tile q (32 cells, 8x4) of a block: Morton bits
+// x0 y0 x1 y1 x2 | y2 x3 y3 x4 y4.
+__host__ __device__ __forceinline__ uint32_t morton_tile_x(uint32_t q) {
+    return 8u * (((q >> 1) & 1u) | ((q >> 2) & 2u));
+}
+__host__ __device__ __forceinline__ int morton_tile_y(uint32_t q) {
+    return 4 * (int)((q & 1u) | ((q >> 1) & 2u) | ((q >> 2) & 4u));
+}
+
+// Cell q of such a tile, x | y << 5.
+__host__ __device__ __forceinline__ uint32_t morton_tile_cell(uint32_t q) {
+    return (q & 1u) | ((q >> 1) & 2u) | ((q >> 2) & 4u) | (((q >> 1) & 1u) << 5) | (((q >> 3) & 1u) << 6);
 }
 
 // Virtual cell (X, Y) -> lattice cell; false for padding (shadergen.cpp:497-503).

@@ -61,75 +61,109 @@ __device__ __forceinline__ float ff_lerp(FF A, FF B, FF t) {
 // Integer lattice index -> float without the conversion pipe (0 <= v < 2^23).
 __device__ __forceinline__ float index_to_float(int v) { return __int_as_float(0x4B000000 | v) - 8388608.0f; }
 
-// The field samples one vertex reads around its edge a -> b = a + e_axis:
-// f(a), f(b), f(a +- e_i), f(b +- e_i).  All loads of a vertex are issued in
-// one branch-free block: interior cells (every sample inside the lattice)
-// through precomputed element offsets, boundary cells with each coordinate
-// clamped (GL_CLAMP + NEAREST), functor fields by evaluating the functor.
-struct EdgeField {
-    float va, vb;
-    float ap[3], bp[3];  // f(a + e_i), f(b + e_i)
-    float am[3], bm[3];  // f(a - e_i), f(b - e_i)   (central differences only)
+// One crossed edge: from lattice point a (its cell's corner, offset g & 7) along
+// `axis` = g >> 3 = u; v, w are the next two axes (cyclically).
+struct EdgeAt {
+    int a[3];
+    int axis;
+    bool interior;      // every sample the vertex reads lies in an array field indexed with 32 bits ...
+    uint32_t at;        // ... the element index of a ...
+    int ou, ov, ow;     // ... and the element strides along u, v, w
 };
 
+// The samples of a cell's edges span cell-1 .. cell+3 on each axis.
+__device__ __forceinline__ bool interior_cell(const Volume& V, int x, int y, int z) {
+    return x >= 1 && x <= V.lattice[0] - 4 && y >= 1 && y <= V.lattice[1] - 4 && z >= 1 && z <= V.lattice[2] - 4;
+}
+
+// {element index of a - that of its cell, strides along u, v, w} of edge geometry g.
+__device__ __forceinline__ int4 edge_strides(const Volume& V, uint32_t g) {
+    const int oy = (int)V.row_pitch, oz = (int)V.slice_pitch, axis = (int)(g >> 3);
+    return make_int4((int)(g & 1u) + (g & 2u ? oy : 0) + (g & 4u ? oz : 0), axis == 0 ? 1 : axis == 1 ? oy : oz,
+                     axis == 0 ? oy : axis == 1 ? oz : 1, axis == 0 ? oz : axis == 1 ? 1 : oy);
+}
+
+// The edge of geometry g of cell (x, y, z).
+__device__ __forceinline__ EdgeAt edge_at(const Volume& V, int x, int y, int z, uint32_t g) {
+    const int4 o = edge_strides(V, g);
+    EdgeAt E;
+    E.a[0] = x + (int)(g & 1u);
+    E.a[1] = y + (int)((g >> 1) & 1u);
+    E.a[2] = z + (int)((g >> 2) & 1u);
+    E.axis = (int)(g >> 3);
+    E.interior = V.idx32 && interior_cell(V, x, y, z);
+    E.at = (uint32_t)z * (uint32_t)V.slice_pitch + (uint32_t)y * (uint32_t)V.row_pitch + (uint32_t)x + (uint32_t)o.x;
+    E.ou = o.y;
+    E.ov = o.z;
+    E.ow = o.w;
+    return E;
+}
+
+// The field samples one vertex reads: f(a), f(b) with b = a + e_u, f(a - e_u),
+// f(b + e_u), f(a +- e_v), ... -- 12 samples for central differences, 7 forward
+// (f(a + e_u) is f(b), f(b - e_u) is f(a)).  All loads of a vertex are issued
+// in one branch-free block: interior cells through element offsets, boundary
+// cells with each coordinate clamped (GL_CLAMP + NEAREST), functor fields by
+// evaluating the functor.
+struct EdgeField {
+    float va, vb;
+    float am, bp;              // f(a - e_u) (central differences only), f(b + e_u)
+    float ap[2], bpv[2];       // f(a + e_v), f(a + e_w); the same at b
+    float amv[2], bmv[2];      // f(a - e_v), f(a - e_w); the same at b (central differences only)
+};
+
+// Component i of a vector given along (u, v, w).
+__device__ __forceinline__ float unrotate(int axis, int i, const float r[3]) {
+    const int at = i - axis;  // -2 .. 2, mod 3 the index along (u, v, w)
+    return at == 0 ? r[0] : (at == 1 || at == -2) ? r[1] : r[2];
+}
+
 template <int FT, bool CENTRAL, class UF = NoUserField>
-__device__ __forceinline__ void gather_edge(const Volume& V, const int* a, int axis, int cx, int cy, int cz,
-                                            EdgeField& F) {
-    const int ex = axis == 0, ey = axis == 1, ez = axis == 2;
+__device__ __forceinline__ void gather_edge(const Volume& V, const EdgeAt& E, EdgeField& F) {
     constexpr bool kArray = FT != kFieldFunctor && FT != kFieldUser;
-    // samples span cell-1 .. cell+3 on each axis
-    const bool interior = kArray && cx >= 1 && cx <= V.lattice[0] - 4 && cy >= 1 && cy <= V.lattice[1] - 4 &&
-                          cz >= 1 && cz <= V.lattice[2] - 4;
-    if (kArray && interior && V.idx32) {
-        // 32-bit element offsets from the sample at a (one wide address each)
+    if (kArray && E.interior) {
         using T = typename std::conditional<
             FT == kFieldF32, float, typename std::conditional<FT == kFieldF32X4, float4, unsigned char>::type>::type;
-        const int o[3] = {1, (int)V.row_pitch, (int)V.slice_pitch};
-        const T* pa = static_cast<const T*>(V.field) + (a[2] * o[2] + a[1] * o[1] + a[0]);
-        const T* pb = pa + (axis == 0 ? o[0] : axis == 1 ? o[1] : o[2]);
-        auto ld = [](const T* p) -> float {
-            if constexpr (FT == kFieldF32) return __ldg(p);
-            else if constexpr (FT == kFieldF32X4) return __ldg(&p->w);
-            else if constexpr (FT == kFieldU8) return u8_to_float(__ldg(p));
-            else return unorm8_to_float(__ldg(p));
+        const T* field = static_cast<const T*>(V.field);
+        auto ld = [&](uint32_t at) -> float {
+            if constexpr (FT == kFieldF32) return __ldg(field + at);
+            else if constexpr (FT == kFieldF32X4) return __ldg(&field[at].w);
+            else if constexpr (FT == kFieldU8) return u8_to_float(__ldg(field + at));
+            else return unorm8_to_float(__ldg(field + at));
         };
+        const uint32_t pa = E.at, pb = E.at + (uint32_t)E.ou;
+        const uint32_t o[2] = {(uint32_t)E.ov, (uint32_t)E.ow};
         F.va = ld(pa);
         F.vb = ld(pb);
+        F.bp = ld(pb + (uint32_t)E.ou);
+        if (CENTRAL) F.am = ld(pa - (uint32_t)E.ou);
 #pragma unroll
-        for (int i = 0; i < 3; i++) {
+        for (int i = 0; i < 2; i++) {
             F.ap[i] = ld(pa + o[i]);
-            F.bp[i] = ld(pb + o[i]);
+            F.bpv[i] = ld(pb + o[i]);
             if (CENTRAL) {
-                F.am[i] = ld(pa - o[i]);
-                F.bm[i] = ld(pb - o[i]);
-            }
-        }
-    } else if (kArray && interior) {
-        const long long o[3] = {1ll, V.row_pitch, V.slice_pitch};
-        const long long pa = (long long)a[2] * V.slice_pitch + (long long)a[1] * V.row_pitch + a[0];
-        const long long pb = pa + (axis == 0 ? o[0] : axis == 1 ? o[1] : o[2]);
-        F.va = fetch_raw<FT>(V, pa);
-        F.vb = fetch_raw<FT>(V, pb);
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-            F.ap[i] = fetch_raw<FT>(V, pa + o[i]);
-            F.bp[i] = fetch_raw<FT>(V, pb + o[i]);
-            if (CENTRAL) {
-                F.am[i] = fetch_raw<FT>(V, pa - o[i]);
-                F.bm[i] = fetch_raw<FT>(V, pb - o[i]);
+                F.amv[i] = ld(pa - o[i]);
+                F.bmv[i] = ld(pb - o[i]);
             }
         }
     } else {
-        F.va = fetch<FT, UF>(V, a[0], a[1], a[2]);
-        F.vb = fetch<FT, UF>(V, a[0] + ex, a[1] + ey, a[2] + ez);
+        const int u[3] = {E.axis == 0, E.axis == 1, E.axis == 2};
+        auto at = [&](int nu, int nv, int nw) {
+            // v is the axis after u, w the one before it
+            return fetch<FT, UF>(V, E.a[0] + nu * u[0] + nv * u[2] + nw * u[1], E.a[1] + nu * u[1] + nv * u[0] + nw * u[2],
+                                 E.a[2] + nu * u[2] + nv * u[1] + nw * u[0]);
+        };
+        F.va = at(0, 0, 0);
+        F.vb = at(1, 0, 0);
+        F.bp = at(2, 0, 0);
+        if (CENTRAL) F.am = at(-1, 0, 0);
 #pragma unroll
-        for (int i = 0; i < 3; i++) {
-            const int dx = i == 0, dy = i == 1, dz = i == 2;
-            F.ap[i] = fetch<FT, UF>(V, a[0] + dx, a[1] + dy, a[2] + dz);
-            F.bp[i] = fetch<FT, UF>(V, a[0] + ex + dx, a[1] + ey + dy, a[2] + ez + dz);
+        for (int i = 0; i < 2; i++) {
+            F.ap[i] = at(0, i == 0, i == 1);
+            F.bpv[i] = at(1, i == 0, i == 1);
             if (CENTRAL) {
-                F.am[i] = fetch<FT, UF>(V, a[0] - dx, a[1] - dy, a[2] - dz);
-                F.bm[i] = fetch<FT, UF>(V, a[0] + ex - dx, a[1] + ey - dy, a[2] + ez - dz);
+                F.amv[i] = at(0, -(i == 0), -(i == 1));
+                F.bmv[i] = at(1, -(i == 0), -(i == 1));
             }
         }
     }
@@ -148,14 +182,13 @@ enum { kGeomForward = 0, kGeomCentral = 1, kGeomBinary = 2 };
 // 7u sqrt(sum_i (|A_i|+|B_i|)^2), u = 2^-24; when that bound exceeds 2e-6 of
 // |n| (a normal that nearly cancels) the vertex is recomputed in float-float.
 template <int FT, int MODE, class UF = NoUserField>
-__device__ __forceinline__ void edge_vertex(const Volume& V, const int* a, int axis, int cx, int cy, int cz,
-                                            const float* binary_normal, float p[3], float n[3], float& t_out) {
+__device__ __forceinline__ void edge_vertex(const Volume& V, const EdgeAt& E, float p[3], float n[3], float& t_out) {
+    const int* a = E.a;
+    const int axis = E.axis;
     float t;
     if (MODE == kGeomBinary) {
         t = 0.5f;
-        n[0] = binary_normal[0];
-        n[1] = binary_normal[1];
-        n[2] = binary_normal[2];
+        n[0] = n[1] = n[2] = 0.0f;  // the caller has the table normal of the vertex's case
     } else if (V.gradient) {
         // gradient mode (shadergen.cpp:539-551): t from the values at a and b,
         // the gradients from HPMC_fetchGrad -- a functor's analytic gradient or
@@ -203,25 +236,22 @@ __device__ __forceinline__ void edge_vertex(const Volume& V, const int* a, int a
             n[i] = (MODE == kGeomCentral) ? -g : iso - g;
         }
     } else {
-        EdgeField F;
-        gather_edge<FT, MODE == kGeomCentral, UF>(V, a, axis, cx, cy, cz, F);
+        EdgeField F{};
+        gather_edge<FT, MODE == kGeomCentral, UF>(V, E, F);
         const float iso = V.iso;
         t = (F.va - iso) / (F.va - F.vb);  // (f(a) - iso) / (f(a) - f(b)), relative error <= 3u
-        float s2 = 0.0f, n2 = 0.0f;
+        float s2 = 0.0f, n2 = 0.0f, r[3];  // r: the normal along (u, v, w)
+        // end-point samples (forward) or differences (central) along u, v, w
+        const float hiA[3] = {F.vb, F.ap[0], F.ap[1]}, hiB[3] = {F.bp, F.bpv[0], F.bpv[1]};
+        const float loA[3] = {F.am, F.amv[0], F.amv[1]}, loB[3] = {F.va, F.bmv[0], F.bmv[1]};
 #pragma unroll
         for (int i = 0; i < 3; i++) {
-            float A, B;
-            if (MODE == kGeomForward) {
-                A = iso - F.ap[i];
-                B = iso - F.bp[i];
-            } else {
-                A = F.ap[i] - F.am[i];
-                B = F.bp[i] - F.bm[i];
-            }
-            n[i] = fmaf(t, B - A, A);
+            const float A = MODE == kGeomForward ? iso - hiA[i] : hiA[i] - loA[i];
+            const float B = MODE == kGeomForward ? iso - hiB[i] : hiB[i] - loB[i];
+            r[i] = fmaf(t, B - A, A);
             const float s = fabsf(A) + fabsf(B);
             s2 = fmaf(s, s, s2);
-            n2 = fmaf(n[i], n[i], n2);
+            n2 = fmaf(r[i], r[i], n2);
         }
         if (s2 > 23.0f * n2) {
             // ill-conditioned: float-float crossing parameter and lerps
@@ -229,16 +259,14 @@ __device__ __forceinline__ void edge_vertex(const Volume& V, const int* a, int a
 #pragma unroll
             for (int i = 0; i < 3; i++) {
                 if (MODE == kGeomForward)
-                    n[i] = ff_lerp(two_sum(iso, -F.ap[i]), two_sum(iso, -F.bp[i]), tf);
+                    r[i] = ff_lerp(two_sum(iso, -hiA[i]), two_sum(iso, -hiB[i]), tf);
                 else
-                    n[i] = ff_lerp(two_sum(F.ap[i], -F.am[i]), two_sum(F.bp[i], -F.bm[i]), tf);
+                    r[i] = ff_lerp(two_sum(hiA[i], -loA[i]), two_sum(hiB[i], -loB[i]), tf);
             }
             t = tf.hi + tf.lo;
         }
-        if (MODE == kGeomCentral) {
 #pragma unroll
-            for (int i = 0; i < 3; i++) n[i] *= -0.5f;
-        }
+        for (int i = 0; i < 3; i++) n[i] = unrotate(axis, i, r) * (MODE == kGeomCentral ? -0.5f : 1.0f);
     }
 #pragma unroll
     for (int i = 0; i < 3; i++) {

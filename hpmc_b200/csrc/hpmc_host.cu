@@ -86,6 +86,7 @@ void volume_layout(Volume& V, const int lattice[3], const int cells[3], const fl
         V.top_cached = (int)end;
     }
     V.column_layout = (2 * V.tile_x >= 32 && 2 * V.tile_y >= 32) ? 1 : 0;
+    V.slot_words = V.column_layout ? kRowSlotWords : kCodeSlotWords;
     V.nfx = (V.cells[0] + 31) / 32;
     V.nfy = (V.cells[1] + 31) / 32;
     V.column_slices = kColumnSliceChoices[3];

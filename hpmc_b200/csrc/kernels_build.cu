@@ -28,17 +28,7 @@ namespace hpmc {
 // box): a column's boxes stream through a TMA ring (each sample leaves HBM
 // once; halo rows/columns are shared with neighbouring columns through L2).
 // The single-volume kernel is persistent (columns from a device queue); the
-// batched one takes one column brick per CTA.  Non-empty blocks store their
-// 1024 codes in Morton order and each 32-cell tile's active mask and vertex
-// count in their arena slot (1.25 KiB), from which a traversal warp builds the
-// block's active-cell list when it enters the block.
-//
-// Measured alternatives for the list: written by the classifier (each
-// non-empty block's serial gathers stall the box barrier: +20 us at 512^3),
-// or by a separate pass over queued slots beside the reduction (issue-bound,
-// ~500 warp instructions per list, not hidden by the 7 us reduction tree:
-// +11 us) -- both slower than one build per warp in the traversal, where the
-// latency of the list's gathers overlaps other warps' vertex work.
+// batched one takes one column brick per CTA.
 template <int FT>
 struct ColumnGeom {
     using T = typename std::conditional<FT == kFieldF32, float, uint8_t>::type;

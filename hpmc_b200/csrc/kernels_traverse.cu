@@ -5,29 +5,25 @@
 // GL3+ path) driven by HPMCextractVertices (triface.cpp:332-457), one
 // invocation per output vertex in batches of 3000 (constants.cpp:198).
 //
-// Here one persistent grid walks the vertex range; a warp owns 32 consecutive
-// vertices per round:
-//   1. descent (warp-cooperative): the warp descends the dense levels for the
-//      first vertex not covered by its cached block, from the top (cached in
-//      shared memory) to the 1024-key block, taking the first child whose
-//      running sum exceeds the key exactly as shadergen.cpp:448-467 does.  All
-//      lanes walk the same path, so every load is one broadcast transaction;
-//      consecutive vertices reuse the block and skip the descent, and a warp
-//      that walks out of its block takes the next non-empty one from the
-//      following 32 level-5 entries (one coalesced load) when it lies there.
-//   2. in-block lookup (warp-cooperative; replaces the base-level steps of
+// Here one persistent grid walks the vertex range, a contiguous range per warp:
+//   1. descent (warp-cooperative): the warp descends the dense levels for its
+//      first vertex, from the top (cached in shared memory) to the 1024-key
+//      block, taking the first child whose running sum exceeds the key exactly
+//      as shadergen.cpp:448-467 does; a warp that walks out of its block takes
+//      the next non-empty one from the following 32 level-5 entries (one
+//      coalesced load) when it lies there.
+//   2. cells (warp-cooperative; replaces the base-level steps of
 //      shadergen.cpp:469-495): the classifier left every non-empty block's
-//      1024 codes in Morton order and, per 32-cell Morton tile, its active
-//      mask and vertex count in the block's arena slot; a warp entering the
-//      block turns them into the block's active-cell list (cells with their
-//      first vertex, in vertex order) in its shared memory with one scan, and
-//      per round a lane's cell is found from that list with one OR-reduction
-//      of the cell starts that fall in the round's window and a popcount (no
-//      per-vertex search).
-//   3. geometry (shadergen.cpp:497-563): edge from the case table, crossing
-//      parameter t, position and normal; FP32 arithmetic with a float-float
-//      fallback for ill-conditioned normals; coalesced streaming float4
-//      stores.
+//      sample bits in the block's arena slot; the warp derives the active
+//      cells in Morton (= vertex) order and takes them 32 at a time, one per
+//      lane: code, vertex count, and one scan for the first vertices.
+//   3. edges: the distinct crossed edges of the 32 cells are numbered, and
+//      each one's vertex -- crossing parameter, position, normal
+//      (shadergen.cpp:497-563) -- is computed once, into shared memory; FP32
+//      arithmetic with a float-float fallback for ill-conditioned normals.
+//   4. vertices: a lane finds its vertex's cell with one OR-reduction and a
+//      popcount, the edge from the case table, and copies the edge's vertex to
+//      the outputs with coalesced streaming float4 stores.
 #include <cuda_runtime.h>
 #include <cstdint>
 
@@ -59,9 +55,119 @@ __device__ __forceinline__ void scatter(const Volume& V, float* dfield, const in
 }
 }  // namespace
 
+// Every distinct edge of a group of cells is differentiated once: the vertices
+// on it -- the same crossing emitted by neighbouring triangles -- have the same
+// Jacobian, so their cotangents are summed into the edge's slot first.  (Summing
+// only within rounds of 32 vertices, with a third of the lanes then gathering
+// and scattering, took 50 us on the 128^3 spheres; this takes 27.)
 template <int FT, int MODE>
-__global__ void __launch_bounds__(kThreads, 4) adjoint_kernel(const __grid_constant__ Volume V,
-                                                              const __grid_constant__ AdjointIO A) {
+struct AdjointVertices {
+    const AdjointIO& A;
+    float (*agg)[6];    // the warp's staging area, one row per lane
+    unsigned long long out;
+
+    __device__ __forceinline__ void run(const CellGroup& G) {
+        const Volume& V = G.V;
+        WarpArea& W = G.W;
+        for (uint32_t i = (uint32_t)G.lane; i < G.nedges; i += 32)
+            W.data[0][i] = W.data[1][i] = W.data[2][i] = make_float2(0.f, 0.f);
+        __syncwarp();
+        const uint32_t n = G.last - G.first;
+#pragma unroll 1
+        for (uint32_t i0 = 0; i0 < n; i0 += 32) {
+            const uint32_t i = i0 + (uint32_t)G.lane;
+            const bool act = i < n;
+            const uint32_t slot = act ? W.slot[i] : 0x10000u | (uint32_t)G.lane;
+            float4 dp = make_float4(0.f, 0.f, 0.f, 0.f), dn = dp;
+            if (act) {
+                const unsigned long long o = out + G.first + i;
+                if (A.dpos) dp = __ldg(A.dpos + o);
+                if (A.dnrm) dn = __ldg(A.dnrm + o);
+            }
+            // lanes on the same edge: the lowest one adds up their cotangents
+            const unsigned int peers = __match_any_sync(0xffffffffu, slot);
+            float* mine = agg[G.lane];
+            mine[0] = dp.x; mine[1] = dp.y; mine[2] = dp.z;
+            mine[3] = dn.x; mine[4] = dn.y; mine[5] = dn.z;
+            __syncwarp();
+            if (act && __ffs((int)peers) - 1 == G.lane) {
+                for (unsigned int rest = peers & (peers - 1u); rest; rest &= rest - 1u) {
+                    const float* q = agg[__ffs((int)rest) - 1];
+                    dp.x += q[0]; dp.y += q[1]; dp.z += q[2];
+                    dn.x += q[3]; dn.y += q[4]; dn.z += q[5];
+                }
+                float2 &s0 = W.data[0][slot], &s1 = W.data[1][slot], &s2 = W.data[2][slot];
+                s0.x += dp.x; s0.y += dp.y; s1.x += dp.z;
+                s1.y += dn.x; s2.x += dn.y; s2.y += dn.z;
+            }
+            __syncwarp();
+        }
+        G.edges([&](uint32_t slot, const EdgeAt& E) {
+            const int ax = E.axis;
+            const float iso = V.iso;
+            const float2 s0 = W.data[0][slot], s1 = W.data[1][slot], s2 = W.data[2][slot];
+            EdgeField F{};
+            gather_edge<FT, MODE == kModeCentral>(V, E, F);
+            // along (u, v, w): the edge's axis and the two after it
+            const float sc[3] = {V.scale[0], V.scale[1], V.scale[2]};
+            const float dp[3] = {s0.x * sc[0], s0.y * sc[1], s1.x * sc[2]};
+            const float dn[3] = {s1.y * sc[0], s2.x * sc[1], s2.y * sc[2]};
+            const float du = ax == 0 ? dn[0] : ax == 1 ? dn[1] : dn[2];
+            const float dvw[2] = {ax == 0 ? dn[1] : ax == 1 ? dn[2] : dn[0], ax == 0 ? dn[2] : ax == 1 ? dn[0] : dn[1]};
+            const int u[3] = {ax == 0, ax == 1, ax == 2};
+            auto add = [&](int nu, int nv, int nw, float g) {
+                if (E.interior) {
+                    atomicAdd(A.dfield + (E.at + (uint32_t)(nu * E.ou + nv * E.ov + nw * E.ow)), g);
+                    return;
+                }
+                scatter(V, A.dfield, E.a, nu * u[0] + nv * u[2] + nw * u[1], nu * u[1] + nv * u[0] + nw * u[2],
+                        nu * u[2] + nv * u[1] + nw * u[0], g);
+            };
+            const float den = F.va - F.vb;
+            const FF tf = ff_ratio_of_diffs(F.va, iso, F.va, F.vb);
+            const float t = tf.hi + tf.lo;
+            const float omt = 1.0f - t;
+            float dLdt = ax == 0 ? dp[0] : ax == 1 ? dp[1] : dp[2];
+            float ga = 0.0f, gb = 0.0f;  // direct contributions to samples a and b
+            if (MODE == kModeForward) {
+                dLdt += du * (F.vb - F.bp);
+                gb -= omt * du;
+                add(2, 0, 0, -t * du);
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    dLdt += dvw[i] * (F.ap[i] - F.bpv[i]);
+                    add(0, i == 0, i == 1, -omt * dvw[i]);
+                    add(1, i == 0, i == 1, -t * dvw[i]);
+                }
+            } else {
+                dLdt -= 0.5f * du * ((F.bp - F.va) - (F.vb - F.am));
+                const float wa = -0.5f * omt * du, wb = -0.5f * t * du;
+                gb += wa;
+                ga -= wb;
+                add(-1, 0, 0, -wa);
+                add(2, 0, 0, wb);
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    dLdt -= 0.5f * dvw[i] * ((F.bpv[i] - F.bmv[i]) - (F.ap[i] - F.amv[i]));
+                    const float va = -0.5f * omt * dvw[i], vb = -0.5f * t * dvw[i];
+                    add(0, i == 0, i == 1, va);
+                    add(0, -(i == 0), -(i == 1), -va);
+                    add(1, i == 0, i == 1, vb);
+                    add(1, -(i == 0), -(i == 1), -vb);
+                }
+            }
+            const float inv = 1.0f / (den * den);
+            ga += dLdt * (iso - F.vb) * inv;
+            gb += dLdt * (F.va - iso) * inv;
+            add(0, 0, 0, ga);
+            add(1, 0, 0, gb);
+        });
+    }
+};
+
+template <int FT, int MODE>
+__global__ void __launch_bounds__(kThreads, kTraverseCtas) adjoint_kernel(const __grid_constant__ Volume V,
+                                                                          const __grid_constant__ AdjointIO A) {
     extern __shared__ __align__(16) uint8_t s_traverse[];
     TraverseSmem& S = *reinterpret_cast<TraverseSmem*>(s_traverse);
     __shared__ float S_agg[kWarps][32][6];  // cotangents of lanes sharing an edge
@@ -69,96 +175,12 @@ __global__ void __launch_bounds__(kThreads, 4) adjoint_kernel(const __grid_const
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned long long total = V.ctrl->total;
     const uint32_t N = (uint32_t)(total < A.count ? total : A.count);
-    const float iso = V.iso;
-    const uint32_t rounds = item_rounds(N, gridDim.x);
-    const uint32_t VW = 32u * rounds;
+    const uint32_t VW = 32u * item_rounds(N, gridDim.x);
     const uint32_t nchunks = (N + VW - 1) / VW;
-    WarpBlock B;
-    B.have = false;
-    B.list = S.list[warp];
-    for (uint32_t chunk = next_chunk(V, lane); chunk < nchunks; chunk = next_chunk(V, lane)) {
-#pragma unroll 1
-        for (uint32_t r = 0; r < rounds; r++) {
-            const uint32_t v = chunk * VW + 32u * r + lane;
-            const bool act = v < N;
-            if (!__any_sync(0xffffffffu, act)) break;
-            VertexCell c;
-            const bool have = resolve_vertex(V, S, lane, v, act, B, c);
-            // Warp aggregation: vertices on the same edge (a, axis) -- the same
-            // crossing emitted by neighbouring triangles -- have the same
-            // Jacobian, so their cotangents are summed first and one lane (the
-            // lowest of the group) scatters once for all of them.
-            EdgeGeom g{};
-            float4 dp = make_float4(0.f, 0.f, 0.f, 0.f), dn = dp;
-            unsigned long long key = ~0ull - (unsigned long long)lane;  // unique for lanes without a vertex
-            if (have) {
-                g = edge_of(S, c);
-                const unsigned long long o = V.vertex_base + v;
-                if (A.dpos) dp = __ldg(A.dpos + o);
-                if (A.dnrm) dn = __ldg(A.dnrm + o);
-                key = ((((unsigned long long)g.a[2] * (unsigned long long)V.lattice[1] + (unsigned long long)g.a[1]) *
-                            (unsigned long long)V.lattice[0] + (unsigned long long)g.a[0]) << 2) | (unsigned)g.axis;
-            }
-            const unsigned int peers = __match_any_sync(0xffffffffu, key);
-            const bool leader = have && (__ffs(peers) - 1 == lane);
-            if (__popc(peers) > 1) {
-                float* slot = S_agg[warp][lane];
-                slot[0] = dp.x; slot[1] = dp.y; slot[2] = dp.z;
-                slot[3] = dn.x; slot[4] = dn.y; slot[5] = dn.z;
-            }
-            __syncwarp();
-            if (leader && __popc(peers) > 1) {
-                unsigned int rest = peers & (peers - 1u);  // the other lanes of the group
-                while (rest) {
-                    const float* q = S_agg[warp][__ffs(rest) - 1];
-                    dp.x += q[0]; dp.y += q[1]; dp.z += q[2];
-                    dn.x += q[3]; dn.y += q[4]; dn.z += q[5];
-                    rest &= rest - 1u;
-                }
-            }
-            __syncwarp();
-            if (!leader) continue;
-            const int ax = g.axis;
-            const int ex = ax == 0, ey = ax == 1, ez = ax == 2;
-            EdgeField F;
-            gather_edge<FT, MODE == kModeCentral>(V, g.a, ax, c.x, c.y, c.z, F);
-            const float dpv[3] = {dp.x, dp.y, dp.z};
-            const float dnv[3] = {dn.x * V.scale[0], dn.y * V.scale[1], dn.z * V.scale[2]};
-            const float va = F.va, vb = F.vb;
-            const float den = va - vb;
-            const FF tf = ff_ratio_of_diffs(va, iso, va, vb);
-            const float t = tf.hi + tf.lo;
-            const float omt = 1.0f - t;
-            float dLdt = dpv[ax] * V.scale[ax];
-            float ga = 0.0f, gb = 0.0f;  // direct contributions to samples a and b
-#pragma unroll
-            for (int i = 0; i < 3; i++) {
-                const int dx = i == 0, dy = i == 1, dz = i == 2;
-                const float fa_p = F.ap[i];
-                const float fb_p = F.bp[i];
-                if (MODE == kModeForward) {
-                    dLdt += dnv[i] * (fa_p - fb_p);
-                    const float wa = -omt * dnv[i], wb = -t * dnv[i];
-                    if (i == ax) gb += wa; else scatter(V, A.dfield, g.a, dx, dy, dz, wa);
-                    scatter(V, A.dfield, g.a, ex + dx, ey + dy, ez + dz, wb);
-                } else {
-                    const float fa_m = F.am[i];
-                    const float fb_m = F.bm[i];
-                    dLdt += -0.5f * dnv[i] * ((fb_p - fb_m) - (fa_p - fa_m));
-                    const float wa = -0.5f * omt * dnv[i], wb = -0.5f * t * dnv[i];
-                    if (i == ax) gb += wa; else scatter(V, A.dfield, g.a, dx, dy, dz, wa);
-                    scatter(V, A.dfield, g.a, -dx, -dy, -dz, -wa);
-                    scatter(V, A.dfield, g.a, ex + dx, ey + dy, ez + dz, wb);
-                    if (i == ax) ga -= wb; else scatter(V, A.dfield, g.a, ex - dx, ey - dy, ez - dz, -wb);
-                }
-            }
-            const float inv = 1.0f / (den * den);
-            ga += dLdt * (iso - vb) * inv;
-            gb += dLdt * (va - iso) * inv;
-            scatter(V, A.dfield, g.a, 0, 0, 0, ga);
-            scatter(V, A.dfield, g.a, ex, ey, ez, gb);
-        }
-    }
+    set_volume(V, S.warp[warp], lane);
+    AdjointVertices<FT, MODE> p{A, S_agg[warp], V.vertex_base};
+    for (uint32_t chunk = next_chunk(V, lane); chunk < nchunks; chunk = next_chunk(V, lane))
+        walk_range(V, S, S.warp[warp], lane, chunk * VW, min(N, (chunk + 1u) * VW), N, p);
     finish_queue(V);
 }
 
@@ -169,55 +191,38 @@ __global__ void __launch_bounds__(kThreads, 4) adjoint_kernel(const __grid_const
 // the descriptors have top_cached = 0, so the descent reads the dense levels
 // through L1 instead of a per-CTA cache.
 template <int FT, int MODE>
-__global__ void __launch_bounds__(kThreads, 4) traverse_batch(const __grid_constant__ BatchDev Bt,
-                                                              const __grid_constant__ TraverseOut O) {
+__global__ void __launch_bounds__(kThreads, kTraverseCtas) traverse_batch(const __grid_constant__ BatchDev Bt,
+                                                                          const __grid_constant__ TraverseOut O) {
     // dynamic: TraverseSmem, then one volume descriptor per warp
     extern __shared__ __align__(16) uint8_t s_traverse[];
     TraverseSmem& S = *reinterpret_cast<TraverseSmem*>(s_traverse);
-    Volume* s_vol = reinterpret_cast<Volume*>(s_traverse + kBatchVolOffset);
     load_base_tables(S);
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t VW = 32u * (uint32_t)Bt.rounds;
     const uint32_t nitems = __ldcg(Bt.chunk_start + Bt.nvol);
-    const Volume& V = s_vol[warp];
+    Volume* const s_vol = reinterpret_cast<Volume*>(s_traverse + sizeof(TraverseSmem) + warp * kVolumeHead);
+    const Volume& V = *s_vol;
     int cur = -1;
     uint32_t c0 = 0, c1 = 0, N = 0;
-    unsigned long long vb = 0;
-    WarpBlock B;
-    B.have = false;
-    B.list = S.list[warp];
+    ExtractVertices<FT, MODE, NoUserField, false> p{O, 0ull};
     for (uint32_t item = next_chunk_batch(Bt, lane); item < nitems; item = next_chunk_batch(Bt, lane)) {
         if (cur < 0 || item < c0 || item >= c1) {
             const int v = find_segment(Bt.chunk_start, Bt.nvol, item);
             __syncwarp();
-            copy_volume(&s_vol[warp], Bt.vols + v, lane, 32);
+            copy_volume(s_vol, Bt.vols + v, lane, 32);
             __syncwarp();
+            set_volume(V, S.warp[warp], lane);
             cur = v;
             c0 = __ldcg(Bt.chunk_start + v);
             c1 = __ldcg(Bt.chunk_start + v + 1);
-            vb = __ldcg(Bt.vbase + v);
+            p.out = __ldcg(Bt.vbase + v);
             const unsigned long long total = __ldcg(&V.ctrl->total);
-            const unsigned long long room = Bt.capacity > vb ? Bt.capacity - vb : 0ull;
+            const unsigned long long room = Bt.capacity > p.out ? Bt.capacity - p.out : 0ull;
             N = (uint32_t)(total < room ? total : room);
-            B.have = false;
         }
         const uint32_t first = (item - c0) * VW;
-#pragma unroll 1
-        for (int r = 0; r < Bt.rounds; r++) {
-            const uint32_t v = first + 32u * r + lane;
-            const bool act = v < N;
-            if (!__any_sync(0xffffffffu, act)) break;
-            VertexCell c;
-            if (!resolve_vertex(V, S, lane, v, act, B, c)) continue;
-            const EdgeGeom g = edge_of(S, c);
-            float p[3], n[3], t;
-            edge_vertex<FT, MODE>(V, g.a, g.axis, c.x, c.y, c.z, g_binary_normals + 3 * (16 * c.code + c.k), p, n,
-                                  t);
-            const unsigned long long o = vb + v;
-            if (O.pos) __stcs(O.pos + o, make_float4(p[0], p[1], p[2], 1.0f));
-            if (O.nrm) __stcs(O.nrm + o, make_float4(n[0], n[1], n[2], 0.0f));
-        }
+        walk_range(V, S, S.warp[warp], lane, first, min(N, first + VW), N, p);
     }
     finish_queue_batch(Bt);
 }
@@ -241,33 +246,45 @@ __device__ __forceinline__ unsigned long long edge_key(const Volume& V, const in
                 (unsigned long long)V.lattice[0] + (unsigned long long)a[0]) * 3ull + (unsigned long long)axis;
 }
 
-__global__ void __launch_bounds__(kThreads, 4) mesh_keys(const __grid_constant__ Volume V, unsigned long long* keys,
-                                                         uint16_t* meta, uint32_t count) {
+struct EdgeKeys {
+    unsigned long long* keys;
+    uint16_t* meta;
+
+    __device__ __forceinline__ void run(const CellGroup& G) {
+        unsigned long long* slots = reinterpret_cast<unsigned long long*>(G.W.data[0]);
+        G.edges([&](uint32_t slot, const EdgeAt& E) { slots[slot] = edge_key(G.V, E.a, E.axis); });
+        const uint32_t n = G.last - G.first;
+        uint32_t c0 = (uint32_t)__ffs((int)G.lanes) - 2u;
+#pragma unroll 1
+        for (uint32_t i0 = 0; i0 < n; i0 += 32) {
+            const uint32_t i = i0 + (uint32_t)G.lane, starts = G.starts(i0);
+            const int c = (int)((c0 + (uint32_t)__popc(starts & (0xffffffffu >> (31 - G.lane)))) & 31u);
+            c0 += (uint32_t)__popc(starts);
+            const uint32_t code = __shfl_sync(0xffffffffu, G.code, c);
+            const uint32_t k = (G.first + i - __shfl_sync(0xffffffffu, G.start, c)) & 15u;
+            if (i >= n) continue;
+            keys[G.first + i] = slots[G.W.slot[i]];
+            meta[G.first + i] = (uint16_t)(code | (k << 8));
+        }
+        __syncwarp();
+    }
+};
+
+__global__ void __launch_bounds__(kThreads, kTraverseCtas) mesh_keys(const __grid_constant__ Volume V,
+                                                                     unsigned long long* keys, uint16_t* meta,
+                                                                     uint32_t count) {
     extern __shared__ __align__(16) uint8_t s_traverse[];
     TraverseSmem& S = *reinterpret_cast<TraverseSmem*>(s_traverse);
     load_tables(V, S);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned long long total = V.ctrl->total;
     const uint32_t N = (uint32_t)(total < count ? total : count);
-    const uint32_t rounds = item_rounds(N, gridDim.x);
-    const uint32_t VW = 32u * rounds;
+    const uint32_t VW = 32u * item_rounds(N, gridDim.x);
     const uint32_t nchunks = (N + VW - 1) / VW;
-    WarpBlock B;
-    B.have = false;
-    B.list = S.list[warp];
-    for (uint32_t chunk = next_chunk(V, lane); chunk < nchunks; chunk = next_chunk(V, lane)) {
-#pragma unroll 1
-        for (uint32_t r = 0; r < rounds; r++) {
-            const uint32_t v = chunk * VW + 32u * r + lane;
-            const bool act = v < N;
-            if (!__any_sync(0xffffffffu, act)) break;
-            VertexCell c;
-            if (!resolve_vertex(V, S, lane, v, act, B, c)) continue;
-            const EdgeGeom g = edge_of(S, c);
-            keys[v] = edge_key(V, g.a, g.axis);
-            meta[v] = (uint16_t)(c.code | (c.k << 8));
-        }
-    }
+    set_volume(V, S.warp[warp], lane);
+    EdgeKeys p{keys, meta};
+    for (uint32_t chunk = next_chunk(V, lane); chunk < nchunks; chunk = next_chunk(V, lane))
+        walk_range(V, S, S.warp[warp], lane, chunk * VW, min(N, (chunk + 1u) * VW), N, p);
     finish_queue(V);
 }
 
@@ -414,7 +431,11 @@ __global__ void __launch_bounds__(kThreads) mesh_emit(const __grid_constant__ Vo
         const uint16_t m = meta[i];
         const int code = m & 0xff, k = (m >> 8) & 15;
         float p[3], nn[3], t;
-        edge_vertex<FT, MODE>(V, a, axis, a[0], a[1], a[2], g_binary_normals + 3 * (16 * code + k), p, nn, t);
+        edge_vertex<FT, MODE>(V, edge_at(V, a[0], a[1], a[2], (uint32_t)axis << 3), p, nn, t);
+        if (MODE == kModeBinary) {
+#pragma unroll
+            for (int c = 0; c < 3; c++) nn[c] = g_binary_normals[3 * (16 * code + k) + c] * V.scale[c];
+        }
         if (pos) pos[u] = make_float4(p[0], p[1], p[2], 1.0f);
         if (nrm) nrm[u] = make_float4(nn[0], nn[1], nn[2], 0.0f);
     }
@@ -423,8 +444,11 @@ __global__ void __launch_bounds__(kThreads) mesh_emit(const __grid_constant__ Vo
 cudaError_t launch_mesh(const Volume& V, const MeshIO& M, int normal_mode, int traverse_grid, int grid,
                         cudaStream_t st) {
     const uint32_t n = M.count;
+    static std::atomic<uint64_t> devices{0};
+    cudaError_t e = allow_traverse_smem(mesh_keys, kTraverseSmem, devices);
+    if (e != cudaSuccess) return e;
     mesh_keys<<<traverse_grid, kThreads, kTraverseSmem, st>>>(V, M.keys, M.meta, n);
-    cudaError_t e = cudaGetLastError();
+    e = cudaGetLastError();
     if (e != cudaSuccess || n == 0) return e;
     if ((e = cudaMemsetAsync(M.table_keys, 0xff, sizeof(unsigned long long) * (M.table_mask + 1ull), st)) !=
             cudaSuccess ||
@@ -463,11 +487,9 @@ cudaError_t launch_traverse(const Volume& V, const TraverseOut& O, int normal_mo
                             cudaStream_t st) {
     const int mode = V.binary ? kModeBinary : (normal_mode == kNormalsCentral ? kModeCentral : kModeForward);
     const bool extra = O.feedback || O.dbg_cell || O.dbg_t;
-#define HPMC_TRAVERSE_LAUNCH(FT_, MODE_)                                                                          \
-    return extra ? launch_dependent(traverse_kernel<FT_, MODE_, NoUserField, true>, grid, kThreads, kTraverseSmem, \
-                                    st, V, O)                                                                     \
-                 : launch_dependent(traverse_kernel<FT_, MODE_, NoUserField, false>, grid, kThreads, kTraverseSmem, \
-                                    st, V, O);
+#define HPMC_TRAVERSE_LAUNCH(FT_, MODE_)                                                 \
+    return extra ? launch_traverse_kernel<FT_, MODE_, NoUserField, true>(V, O, grid, st) \
+                 : launch_traverse_kernel<FT_, MODE_, NoUserField, false>(V, O, grid, st);
 #define HPMC_TRAVERSE_CASE(FT_)                                             \
     case FT_:                                                               \
         if (mode == kModeBinary) HPMC_TRAVERSE_LAUNCH(FT_, kModeBinary)     \
@@ -485,101 +507,74 @@ cudaError_t launch_traverse(const Volume& V, const TraverseOut& O, int normal_mo
 #undef HPMC_TRAVERSE_LAUNCH
 }
 
-cudaError_t launch_adjoint(const Volume& V, const AdjointIO& A, int normal_mode, int grid, cudaStream_t st) {
-    const bool central = normal_mode == kNormalsCentral;
-    // the adjoint's static cotangent buffer plus the traversal's dynamic
-    // shared memory pass the 48 KB a launch gets without opting in
-    static const bool opted_in = [] {
-        const int bytes = (int)kTraverseSmem;
-        cudaFuncSetAttribute(adjoint_kernel<kFieldF32, kModeCentral>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        cudaFuncSetAttribute(adjoint_kernel<kFieldF32, kModeForward>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        cudaFuncSetAttribute(adjoint_kernel<kFieldU8, kModeCentral>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        cudaFuncSetAttribute(adjoint_kernel<kFieldU8, kModeForward>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        cudaFuncSetAttribute(adjoint_kernel<kFieldUNorm8, kModeCentral>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             bytes);
-        cudaFuncSetAttribute(adjoint_kernel<kFieldUNorm8, kModeForward>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             bytes);
-        return true;
-    }();
-    (void)opted_in;
-    switch (V.ftype) {
-        case kFieldF32:
-            if (central) adjoint_kernel<kFieldF32, kModeCentral><<<grid, kThreads, kTraverseSmem, st>>>(V, A);
-            else adjoint_kernel<kFieldF32, kModeForward><<<grid, kThreads, kTraverseSmem, st>>>(V, A);
-            break;
-        case kFieldU8:
-            if (central) adjoint_kernel<kFieldU8, kModeCentral><<<grid, kThreads, kTraverseSmem, st>>>(V, A);
-            else adjoint_kernel<kFieldU8, kModeForward><<<grid, kThreads, kTraverseSmem, st>>>(V, A);
-            break;
-        case kFieldUNorm8:
-            if (central) adjoint_kernel<kFieldUNorm8, kModeCentral><<<grid, kThreads, kTraverseSmem, st>>>(V, A);
-            else adjoint_kernel<kFieldUNorm8, kModeForward><<<grid, kThreads, kTraverseSmem, st>>>(V, A);
-            break;
-        default:
-            return cudaErrorInvalidValue;
-    }
+template <int FT, int MODE>
+static cudaError_t launch_adjoint_kernel(const Volume& V, const AdjointIO& A, int grid, cudaStream_t st) {
+    static std::atomic<uint64_t> devices{0};
+    const cudaError_t e = allow_traverse_smem(adjoint_kernel<FT, MODE>, kTraverseSmem, devices);
+    if (e != cudaSuccess) return e;
+    adjoint_kernel<FT, MODE><<<grid, kThreads, kTraverseSmem, st>>>(V, A);
     return cudaGetLastError();
 }
 
-// The batched traversal needs more than the default 48 KB of dynamic shared memory.
-static void configure_batch_smem() {
-    static bool done = false;
-    if (done) return;
-    done = true;
-    const int bytes = (int)kBatchSmem;
-    cudaFuncSetAttribute(traverse_batch<kFieldF32, kModeCentral>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(traverse_batch<kFieldF32, kModeForward>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(traverse_batch<kFieldU8, kModeCentral>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(traverse_batch<kFieldU8, kModeForward>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(traverse_batch<kFieldUNorm8, kModeCentral>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         bytes);
-    cudaFuncSetAttribute(traverse_batch<kFieldUNorm8, kModeForward>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         bytes);
+cudaError_t launch_adjoint(const Volume& V, const AdjointIO& A, int normal_mode, int grid, cudaStream_t st) {
+    const bool central = normal_mode == kNormalsCentral;
+    switch (V.ftype) {
+        case kFieldF32:
+            return central ? launch_adjoint_kernel<kFieldF32, kModeCentral>(V, A, grid, st)
+                           : launch_adjoint_kernel<kFieldF32, kModeForward>(V, A, grid, st);
+        case kFieldU8:
+            return central ? launch_adjoint_kernel<kFieldU8, kModeCentral>(V, A, grid, st)
+                           : launch_adjoint_kernel<kFieldU8, kModeForward>(V, A, grid, st);
+        case kFieldUNorm8:
+            return central ? launch_adjoint_kernel<kFieldUNorm8, kModeCentral>(V, A, grid, st)
+                           : launch_adjoint_kernel<kFieldUNorm8, kModeForward>(V, A, grid, st);
+        default:
+            return cudaErrorInvalidValue;
+    }
+}
+
+template <int FT, int MODE>
+static cudaError_t launch_batch_kernel(const BatchDev& B, const TraverseOut& O, int grid, cudaStream_t st) {
+    static std::atomic<uint64_t> devices{0};
+    const cudaError_t e = allow_traverse_smem(traverse_batch<FT, MODE>, kBatchSmem, devices);
+    if (e != cudaSuccess) return e;
+    traverse_batch<FT, MODE><<<grid, kThreads, kBatchSmem, st>>>(B, O);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_traverse_batch(const BatchDev& B, const TraverseOut& O, int ftype, int normal_mode, int grid,
                                   cudaStream_t st) {
-    configure_batch_smem();  // set before any capture: the first call comes from traverse_batch_blocks_per_sm
     const bool central = normal_mode == kNormalsCentral;
     switch (ftype) {
         case kFieldF32:
-            if (central) traverse_batch<kFieldF32, kModeCentral><<<grid, kThreads, kBatchSmem, st>>>(B, O);
-            else traverse_batch<kFieldF32, kModeForward><<<grid, kThreads, kBatchSmem, st>>>(B, O);
-            break;
+            return central ? launch_batch_kernel<kFieldF32, kModeCentral>(B, O, grid, st)
+                           : launch_batch_kernel<kFieldF32, kModeForward>(B, O, grid, st);
         case kFieldU8:
-            if (central) traverse_batch<kFieldU8, kModeCentral><<<grid, kThreads, kBatchSmem, st>>>(B, O);
-            else traverse_batch<kFieldU8, kModeForward><<<grid, kThreads, kBatchSmem, st>>>(B, O);
-            break;
+            return central ? launch_batch_kernel<kFieldU8, kModeCentral>(B, O, grid, st)
+                           : launch_batch_kernel<kFieldU8, kModeForward>(B, O, grid, st);
         case kFieldUNorm8:
-            if (central) traverse_batch<kFieldUNorm8, kModeCentral><<<grid, kThreads, kBatchSmem, st>>>(B, O);
-            else traverse_batch<kFieldUNorm8, kModeForward><<<grid, kThreads, kBatchSmem, st>>>(B, O);
-            break;
+            return central ? launch_batch_kernel<kFieldUNorm8, kModeCentral>(B, O, grid, st)
+                           : launch_batch_kernel<kFieldUNorm8, kModeForward>(B, O, grid, st);
         default:
             return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 
-int traverse_batch_blocks_per_sm() {
-    configure_batch_smem();
+// Resident CTAs per SM of one kernel with `bytes` of dynamic shared memory.
+template <class K>
+static int resident_ctas(K* kernel, size_t bytes) {
+    static std::atomic<uint64_t> devices{0};
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, traverse_batch<kFieldF32, kModeCentral>, kThreads,
-                                                      kBatchSmem) !=
-            cudaSuccess ||
-        n < 1)
+    if (allow_traverse_smem(kernel, bytes, devices) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kThreads, bytes) != cudaSuccess || n < 1)
         n = 1;
     return n;
 }
+
+int traverse_batch_blocks_per_sm() { return resident_ctas(traverse_batch<kFieldF32, kModeCentral>, kBatchSmem); }
 
 int traverse_blocks_per_sm() {
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, traverse_kernel<kFieldF32, kModeCentral>, kThreads,
-                                                      kTraverseSmem) !=
-            cudaSuccess ||
-        n < 1)
-        n = 1;
-    return n;
+    return resident_ctas(traverse_kernel<kFieldF32, kModeCentral, NoUserField, false>, kTraverseSmem);
 }
 
 }  // namespace hpmc
-

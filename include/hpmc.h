@@ -292,7 +292,7 @@ int HPMCgetClassifyPath(struct HPMCHistoPyramid* h, int* path);
  * table under a name makes that name valid for HPMCsetFieldCustom.  The
  * table is copied; the functions it points to must stay loaded while handles
  * use the name.  Names starting with "hpmc:" are reserved. */
-#define HPMC_FIELD_FUNCTOR_ABI 1u
+#define HPMC_FIELD_FUNCTOR_ABI 2u
 typedef struct HPMCFieldFunctorOps {
     unsigned int abi;   /* HPMC_FIELD_FUNCTOR_ABI */
     int volume_bytes;   /* size of the volume descriptor the functor was compiled against */

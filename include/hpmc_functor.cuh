@@ -72,13 +72,9 @@ int user_traverse(const void* volume, const void* outputs, int mode, int grid, v
     const Volume& V = *static_cast<const Volume*>(volume);
     const TraverseOut& O = *static_cast<const TraverseOut*>(outputs);
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
-    cudaError_t e;
-    if (mode == kModeBinary)
-        e = launch_dependent(traverse_kernel<kFieldUser, kModeBinary, F>, grid, kThreads, kTraverseSmem, st, V, O);
-    else if (mode == kModeCentral)
-        e = launch_dependent(traverse_kernel<kFieldUser, kModeCentral, F>, grid, kThreads, kTraverseSmem, st, V, O);
-    else
-        e = launch_dependent(traverse_kernel<kFieldUser, kModeForward, F>, grid, kThreads, kTraverseSmem, st, V, O);
+    const cudaError_t e = mode == kModeBinary    ? launch_traverse_kernel<kFieldUser, kModeBinary, F, true>(V, O, grid, st)
+                          : mode == kModeCentral ? launch_traverse_kernel<kFieldUser, kModeCentral, F, true>(V, O, grid, st)
+                                                 : launch_traverse_kernel<kFieldUser, kModeForward, F, true>(V, O, grid, st);
     return e == cudaSuccess ? HPMC_OK : HPMC_ERR_CUDA;
 }
 
