@@ -57,8 +57,8 @@ struct HPMCBatch {
     std::vector<Volume> hv;            // descriptors (device pointers filled in)
     std::vector<uint8_t> column;       // volume uses the TMA column classifier
     std::vector<CUtensorMap> tmaps;
-    std::vector<uint32_t> brick_start, reduce_start;
-    unsigned int bricks = 0, reduce_chunks = 0;
+    std::vector<uint32_t> brick_start, direct_start, reduce_start;
+    unsigned int bricks = 0, direct_bricks = 0, reduce_chunks = 0;
     // device
     unsigned char* d_base = nullptr;
     BatchCtrl* d_bctrl = nullptr;
@@ -66,6 +66,7 @@ struct HPMCBatch {
     Volume* d_vols = nullptr;
     CUtensorMap* d_tmaps = nullptr;
     uint32_t* d_brick_start = nullptr;
+    uint32_t* d_direct_start = nullptr;
     uint32_t* d_reduce_start = nullptr;
     uint32_t* d_chunk_start = nullptr;
     unsigned long long* d_vbase = nullptr;
@@ -101,7 +102,7 @@ void release(HPMCBatch* b) {
     b->d_base = nullptr;
 }
 
-// Column depth of every volume and the brick prefix array.
+// Column depth of every volume and the brick prefix arrays.
 void apply_column_slices(HPMCBatch* b) {
     int zc = b->column_slices;
     if (zc == 0) {
@@ -111,22 +112,27 @@ void apply_column_slices(HPMCBatch* b) {
         for (int c : hpmc::kColumnSliceChoices) {
             long long n = 0;
             for (int v = 0; v < b->nvol; v++)
-                if (b->column[v]) n += (long long)b->hv[v].nfx * b->hv[v].nfy * ((b->hv[v].cells[2] + c - 1) / c);
+                if (b->hv[v].column_layout) n += (long long)b->hv[v].nfx * b->hv[v].nfy * ((b->hv[v].cells[2] + c - 1) / c);
             if (n >= target) {
                 zc = c;
                 break;
             }
         }
     }
-    uint32_t acc = 0;
+    uint32_t acc = 0, direct = 0;
     for (int v = 0; v < b->nvol; v++) {
         Volume& V = b->hv[v];
         V.column_slices = zc;
         b->brick_start[v] = acc;
-        if (b->column[v]) acc += (uint32_t)(V.nfx * V.nfy * ((V.cells[2] + zc - 1) / zc));
+        b->direct_start[v] = direct;
+        const uint32_t columns = (uint32_t)(V.nfx * V.nfy * ((V.cells[2] + zc - 1) / zc));
+        if (b->column[v]) acc += columns;
+        else direct += V.column_layout ? columns : (uint32_t)V.nblocks;
     }
     b->brick_start[b->nvol] = acc;
+    b->direct_start[b->nvol] = direct;
     b->bricks = acc;
+    b->direct_bricks = direct;
     b->upload = true;
 }
 
@@ -147,6 +153,7 @@ BatchDev device_view(const HPMCBatch* b, size_t cap) {
     B.vols = b->d_vols;
     B.tmaps = b->d_tmaps;
     B.brick_start = b->d_brick_start;
+    B.direct_start = b->d_direct_start;
     B.reduce_start = b->d_reduce_start;
     B.vbase = b->d_vbase;
     B.chunk_start = b->d_chunk_start;
@@ -160,10 +167,7 @@ BatchDev device_view(const HPMCBatch* b, size_t cap) {
 // The launches of one batched extraction, on `st` (captured into the graph).
 cudaError_t issue(HPMCBatch* b, float* pos, float* nrm, size_t cap, int traverse_grid, cudaStream_t st) {
     const BatchDev B = device_view(b, cap);
-    const int num_sms = b->constants->num_sms;
-    cudaError_t e = cudaSuccess;
-    for (int v = 0; v < b->nvol && e == cudaSuccess; v++)
-        if (!b->column[v]) e = hpmc::launch_classify(b->hv[v], nullptr, num_sms * 16, st);
+    cudaError_t e = hpmc::launch_classify_batch_direct(B, b->ftype, b->direct_bricks, st);
     if (e == cudaSuccess) e = hpmc::launch_classify_batch(B, b->ftype, b->bricks, st);
     if (e == cudaSuccess) e = hpmc::launch_reduce_batch(B, b->reduce_chunks, st);
     if (e == cudaSuccess) {
@@ -184,6 +188,7 @@ int upload(HPMCBatch* b, cudaStream_t st) {
         cudaMemcpyAsync(b->d_tmaps, b->tmaps.data(), sizeof(CUtensorMap) * b->nvol, cudaMemcpyHostToDevice, st) !=
             cudaSuccess ||
         cudaMemcpyAsync(b->d_brick_start, b->brick_start.data(), n1, cudaMemcpyHostToDevice, st) != cudaSuccess ||
+        cudaMemcpyAsync(b->d_direct_start, b->direct_start.data(), n1, cudaMemcpyHostToDevice, st) != cudaSuccess ||
         cudaMemcpyAsync(b->d_reduce_start, b->reduce_start.data(), n1, cudaMemcpyHostToDevice, st) != cudaSuccess) {
         cudaGetLastError();
         return HPMC_ERR_CUDA;
@@ -259,6 +264,7 @@ int HPMCcreateBatch(HPMCConstants* c, const HPMCBatchVolume* volumes, int count,
     b->column.assign(count, 0);
     b->tmaps.assign(count, CUtensorMap{});
     b->brick_start.assign(count + 1, 0);
+    b->direct_start.assign(count + 1, 0);
     b->reduce_start.assign(count + 1, 0);
 
     // per-volume layouts and sizes
@@ -334,6 +340,8 @@ int HPMCcreateBatch(HPMCConstants* c, const HPMCBatchVolume* volumes, int count,
     off = align_up(off + sizeof(CUtensorMap) * count, 256);
     const size_t o_brick = off;
     off = align_up(off + sizeof(uint32_t) * (count + 1), 256);
+    const size_t o_direct = off;
+    off = align_up(off + sizeof(uint32_t) * (count + 1), 256);
     const size_t o_red = off;
     off = align_up(off + sizeof(uint32_t) * (count + 1), 256);
     const size_t o_chunk = off;
@@ -360,6 +368,7 @@ int HPMCcreateBatch(HPMCConstants* c, const HPMCBatchVolume* volumes, int count,
     b->d_vols = reinterpret_cast<Volume*>(b->d_base + o_vols);
     b->d_tmaps = reinterpret_cast<CUtensorMap*>(b->d_base + o_tmaps);
     b->d_brick_start = reinterpret_cast<uint32_t*>(b->d_base + o_brick);
+    b->d_direct_start = reinterpret_cast<uint32_t*>(b->d_base + o_direct);
     b->d_reduce_start = reinterpret_cast<uint32_t*>(b->d_base + o_red);
     b->d_chunk_start = reinterpret_cast<uint32_t*>(b->d_base + o_chunk);
     b->d_vbase = reinterpret_cast<unsigned long long*>(b->d_base + o_vbase);

@@ -273,6 +273,11 @@ __device__ __forceinline__ uint32_t row_mask(const Volume& V, int x0, int y0, in
 template <int FT>
 using SampleT = typename std::conditional<FT == kFieldU8 || FT == kFieldUNorm8, uint8_t, float>::type;
 
+// Resident direct-classifier CTAs per SM the registers are held to: 3 against
+// 2, 4, 5 measured on whole calls: f32 301x257x129 45.7 us (48.8, 45.4, 48.2),
+// cubic functor 128^3 56.1 (56.2, 60.7, 59.6).
+constexpr int kDirectCtas = 3;
+
 // One sample of an array field, (x, y, z) inside the lattice.
 template <int FT>
 __device__ __forceinline__ SampleT<FT> direct_sample(const Volume& V, int x, int y, int z) {
@@ -283,22 +288,43 @@ __device__ __forceinline__ SampleT<FT> direct_sample(const Volume& V, int x, int
         return fetch_raw<FT>(V, at);
 }
 
-// The lane's samples of the box whose first layer is lattice layer z; indices
-// past the lattice are clamped (their cells are outside the grid and masked).
+// Bit rows of a box of an array field whose first layer is lattice layer z,
+// straight from global memory, four layers of loads at a time; indices past the
+// lattice are clamped (their cells are outside the grid and masked).
 template <int FT>
-__device__ __forceinline__ void load_box_direct(const Volume& V, int x0, int y0, int z, uint32_t gl0, int warp, int lane,
-                                                BoxSamples<SampleT<FT>>& s) {
+__device__ __forceinline__ void direct_box_bits(const Volume& V, int x0, int y0, int z, int nl, uint32_t gl0, float iso,
+                                                int warp, int lane, ColumnBits& C) {
+    constexpr int kHalf = kLayersPerBox / 2;
     const int mx = V.lattice[0] - 1, my = V.lattice[1] - 1, mz = V.lattice[2] - 1;
     const int x = min(x0 + lane, mx), x32 = min(x0 + 32, mx), y32 = min(y0 + 32, my);
+    const uint32_t g0 = gl0 & (kRowBuffers - 1);
+    const int le = edge_layer(gl0, warp), ze = min(z + le, mz);
+    const SampleT<FT> row = direct_sample<FT>(V, x, y32, ze), col = direct_sample<FT>(V, x32, min(y0 + lane, my), ze),
+                      corner = direct_sample<FT>(V, x32, y32, ze);
 #pragma unroll
-    for (int l = 0; l < kLayersPerBox; l++)
+    for (int h = 0; h < 2; h++) {
+        if (h * kHalf >= nl) break;
+        SampleT<FT> v[kHalf][4];
 #pragma unroll
-        for (int i = 0; i < 4; i++)
-            s.v[l][i] = direct_sample<FT>(V, x, min(y0 + 4 * warp + i, my), min(z + l, mz));
-    const int ze = min(z + edge_layer(gl0, warp), mz);
-    s.row = direct_sample<FT>(V, x, y32, ze);
-    s.col = direct_sample<FT>(V, x32, min(y0 + lane, my), ze);
-    s.corner = direct_sample<FT>(V, x32, y32, ze);
+        for (int l = 0; l < kHalf; l++)
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                v[l][i] = direct_sample<FT>(V, x, min(y0 + 4 * warp + i, my), min(z + h * kHalf + l, mz));
+#pragma unroll
+        for (int l = 0; l < kHalf; l++) {
+            uint32_t b[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) b[i] = __ballot_sync(0xffffffffu, below(v[l][i], iso, V.u8_thr));
+            if (h * kHalf + l < nl && lane == 0)
+                *reinterpret_cast<uint4*>(&C.rows[g0 + h * kHalf + l][4 * warp]) = make_uint4(b[0], b[1], b[2], b[3]);
+        }
+    }
+    const uint32_t r32 = __ballot_sync(0xffffffffu, below(row, iso, V.u8_thr));
+    const uint32_t c32 = __ballot_sync(0xffffffffu, below(col, iso, V.u8_thr));
+    if (le < nl && lane == 0) {
+        C.rows[g0 + (uint32_t)le][32] = r32;
+        C.col[g0 + (uint32_t)le] = (uint64_t)c32 | ((uint64_t)below(corner, iso, V.u8_thr) << 32);
+    }
 }
 
 // Bit rows of a box of a functor field: box_bits with every sample evaluated
@@ -339,20 +365,22 @@ __device__ __forceinline__ void functor_box_bits(const Volume& V, int x0, int y0
 // Direct column classifier: column layouts whose field no tensor map covers --
 // rows that are no multiple of 16 bytes, float4 fields, functors.  One CTA per
 // column.  Array samples come straight into registers (one coalesced row per
-// load) and the next box's loads are issued before the current box's slices
-// are classified; functors are evaluated once per sample.  The block
+// load, 16 in flight per lane: keeping a whole next box in registers as well
+// leaves room for 2 CTAs per SM only); functors are evaluated once per sample.  The block
 // classifier it takes over from loads or evaluates 18 samples per 4 cells and
 // visits the padding blocks of the layout.  Kernel times, block classifier ->
-// this one: f32 301x257x129 51.9 -> 19.9 us, UNORM8 253x231x197 62.6 -> 29.1,
-// float4 128^3 18.1 -> 10.5, the cubic functor at 128^3 44.7 -> 16.4.  Issue-
+// this one: f32 301x257x129 51.9 -> 17.9 us, UNORM8 253x231x197 62.6 -> 23.7,
+// float4 128^3 18.1 -> 10.5, the cubic functor at 128^3 44.7 -> 14.3.  Issue-
 // bound on array fields (ballots and slice classification), not by memory.
-template <int FT, class UF = NoUserField>
-__global__ void __launch_bounds__(kThreads, 2) classify_columns_direct(const __grid_constant__ Volume V) {
+//
+// CTA body: column `u` (footprint-fastest) of V.  WAIT: also wait for the
+// previous grid before the field and the pyramid are touched.
+template <int FT, class UF, bool WAIT>
+__device__ __forceinline__ void classify_column_direct(const Volume& V, int u, ColumnBits& C) {
     constexpr bool kArray = FT != kFieldFunctor && FT != kFieldUser;
-    __shared__ __align__(16) ColumnBits C;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int per_slab = V.nfx * V.nfy;
-    const int zc = blockIdx.x / per_slab, r = blockIdx.x - zc * per_slab;
+    const int zc = u / per_slab, r = u - zc * per_slab;
     const int fy = r / V.nfx, fx = r - fy * V.nfx;
     const int x0 = fx * 32, y0 = fy * 32, z0 = zc * V.column_slices;
     const int z1 = min(V.cells[2], z0 + V.column_slices);
@@ -362,20 +390,20 @@ __global__ void __launch_bounds__(kThreads, 2) classify_columns_direct(const __g
     const uint32_t fm = footprint_morton(fx, fy);
     const uint32_t vmask = row_mask(V, x0, y0, lane);
     const bool full = __all_sync(0xffffffffu, vmask == 0xffffffffu);
-    wait_prior_grid();  // the field and the pyramid only after the previous grid
-    BoxSamples<SampleT<FT>> s;
-    if constexpr (kArray) load_box_direct<FT>(V, x0, y0, z0, 0u, warp, lane, s);
+    if (WAIT) wait_prior_grid();
     for (int lb = 0; lb < nlayers; lb += kLayersPerBox) {
         const int nl = min(kLayersPerBox, nlayers - lb);
-        if constexpr (kArray) box_bits(s, nl, (uint32_t)lb, iso, V.u8_thr, warp, lane, C);
+        if constexpr (kArray) direct_box_bits<FT>(V, x0, y0, z0 + lb, nl, (uint32_t)lb, iso, warp, lane, C);
         else functor_box_bits<FT, UF>(V, x0, y0, z0 + lb, nl, (uint32_t)lb, iso, warp, lane, C);
         __syncthreads();  // bit rows of this box ready, and every slice of the box before the last classified
-        if constexpr (kArray) {
-            if (lb + kLayersPerBox < nlayers)
-                load_box_direct<FT>(V, x0, y0, z0 + lb + kLayersPerBox, (uint32_t)(lb + kLayersPerBox), warp, lane, s);
-        }
         classify_box_slices(V, z0, fx, fy, fm, lb, nl, 0u, warp, lane, vmask, full, C);
     }
+}
+
+template <int FT, class UF = NoUserField>
+__global__ void __launch_bounds__(kThreads, kDirectCtas) classify_columns_direct(const __grid_constant__ Volume V) {
+    __shared__ __align__(16) ColumnBits C;
+    classify_column_direct<FT, UF, true>(V, blockIdx.x, C);
 }
 
 // Columns of a volume (the direct classifier's grid).

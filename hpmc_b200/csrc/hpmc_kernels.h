@@ -40,7 +40,8 @@ struct BatchCtrl {
 struct BatchDev {
     const Volume* vols;            // per-volume descriptors (top_cached = 0)
     const CUtensorMap* tmaps;      // per-volume column tensor maps (64-byte aligned)
-    const uint32_t* brick_start;   // nvol + 1: column bricks before volume v
+    const uint32_t* brick_start;   // nvol + 1: column bricks before volume v (volumes with a tensor map)
+    const uint32_t* direct_start;  // nvol + 1: columns or blocks before volume v (the other volumes)
     const uint32_t* reduce_start;  // nvol + 1: reduction chunks before volume v
     unsigned long long* vbase;     // nvol + 1: first output vertex of volume v (written by the reduction)
     uint32_t* chunk_start;         // nvol + 1: traversal work items before volume v (written by the reduction)
@@ -73,6 +74,7 @@ cudaError_t launch_mesh(const Volume& V, const MeshIO& M, int normal_mode, int t
                         cudaStream_t st);
 cudaError_t launch_classify(const Volume& V, const CUtensorMap* tmap, int max_ctas, cudaStream_t st);
 cudaError_t launch_classify_batch(const BatchDev& B, int ftype, unsigned int bricks, cudaStream_t st);
+cudaError_t launch_classify_batch_direct(const BatchDev& B, int ftype, unsigned int bricks, cudaStream_t st);
 cudaError_t launch_reduce_batch(const BatchDev& B, unsigned int chunks, cudaStream_t st);
 cudaError_t launch_traverse_batch(const BatchDev& B, const TraverseOut& O, int ftype, int normal_mode, int grid,
                                   cudaStream_t st);

@@ -422,8 +422,9 @@ __global__ void copy_total(const __grid_constant__ Volume V) {
 }
 
 // ---------------------------------------------------------------------------
-// Batched build.  One classify launch covers the column bricks of every
-// volume (CTA = one brick, its volume found in the brick prefix array); one
+// Batched build.  One classify launch covers the column bricks of every volume
+// with a tensor map (CTA = one brick, its volume found in the brick prefix
+// array), one the bricks of the others; one
 // reduce launch covers the reduction chunks of every volume (each volume's
 // pyramid finished by its own last CTA), and the CTA that completes the last
 // volume scans the per-volume counts into output offsets and traversal work
@@ -441,6 +442,24 @@ __global__ void __launch_bounds__(kThreads) classify_batch_tma(const __grid_cons
     const int fy = (int)(r / (uint32_t)sV.nfx);
     const int fx = (int)(r - (uint32_t)fy * (uint32_t)sV.nfx);
     classify_column_body<FT>(B.tmaps + v, sV, fx, fy, zc);
+}
+
+// The bricks of the volumes without a tensor map, one per CTA: columns (direct
+// classifier) or, for narrow tiles, 32x32 blocks.  One launch for all of them:
+// a launch per volume leaves the GPU nearly empty for about 5 us each (24 byte
+// volumes of edge 20..120: 23 launches, 128 us in all; this one 15 us).
+template <int FT>
+__global__ void __launch_bounds__(kThreads, kDirectCtas) classify_batch_direct(const __grid_constant__ BatchDev B) {
+    __shared__ __align__(16) Volume sV;
+    __shared__ __align__(16) ColumnBits C;
+    __shared__ uint32_t s_warp[kWarps];
+    const int v = find_segment(B.direct_start, B.nvol, blockIdx.x);
+    copy_volume(&sV, B.vols + v, threadIdx.x, blockDim.x);
+    C.cnt[threadIdx.x] = c_vertex_count[threadIdx.x];
+    __syncthreads();
+    const uint32_t u = blockIdx.x - __ldg(B.direct_start + v);
+    if (sV.column_layout) classify_column_direct<FT, NoUserField, false>(sV, (int)u, C);
+    else classify_block_body<FT>(sV, u, C.cnt, s_warp);
 }
 
 namespace {
@@ -614,6 +633,19 @@ cudaError_t launch_classify_batch(const BatchDev& B, int ftype, unsigned int bri
         classify_batch_tma<kFieldU8><<<bricks, kThreads, kRingBytesU8, st>>>(B);
     else if (ftype == kFieldUNorm8)
         classify_batch_tma<kFieldUNorm8><<<bricks, kThreads, kRingBytesU8, st>>>(B);
+    else
+        return cudaErrorInvalidValue;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_classify_batch_direct(const BatchDev& B, int ftype, unsigned int bricks, cudaStream_t st) {
+    if (!bricks) return cudaSuccess;
+    if (ftype == kFieldF32)
+        classify_batch_direct<kFieldF32><<<bricks, kThreads, 0, st>>>(B);
+    else if (ftype == kFieldU8)
+        classify_batch_direct<kFieldU8><<<bricks, kThreads, 0, st>>>(B);
+    else if (ftype == kFieldUNorm8)
+        classify_batch_direct<kFieldUNorm8><<<bricks, kThreads, 0, st>>>(B);
     else
         return cudaErrorInvalidValue;
     return cudaGetLastError();
