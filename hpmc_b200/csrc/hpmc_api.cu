@@ -89,6 +89,7 @@ struct HPMCHistoPyramid {
     int nsets = 0;
     int set = 0;                   // the set of the last build
     Ctrl* d_ctrl = nullptr;
+    hpmc::HostCount* host = nullptr;  // where builds leave their count (mapped host memory), or null
     // the last extraction's outputs (byte ranges), stream and set: the next
     // build overlaps it only on the same stream, into the other set, and with
     // a field that is none of those outputs
@@ -141,6 +142,8 @@ void release_device(HPMCHistoPyramid* h) {
     cudaFree(h->d_levels);
     cudaFree(h->d_arena);
     cudaFree(h->d_ctrl);
+    hpmc::host::give_host_slot(h->host);
+    h->host = nullptr;
     h->d_levels = nullptr;
     h->d_arena = nullptr;
     h->d_ctrl = nullptr;
@@ -220,6 +223,8 @@ bool setup(HPMCHistoPyramid* h) {
             h->status = HPMC_ERR_OUT_OF_MEMORY;
             return false;
         }
+        static_assert(sizeof(hpmc::HostCount) <= 64, "a host slot holds it");
+        h->host = static_cast<hpmc::HostCount*>(hpmc::host::take_host_slot());
         h->levels_cap = (size_t)levels_total;
         h->arena_cap = arena_words;
         h->nsets = nsets;
@@ -235,6 +240,7 @@ bool setup(HPMCHistoPyramid* h) {
     V.arena = h->d_arena;
     V.arena_slots = slots;
     V.ctrl = h->d_ctrl;
+    V.host = h->host;
     h->set = 0;
     h->tainted = false;
     h->built = false;
@@ -289,6 +295,18 @@ int launch_extract(HPMCTraversalHandle* th, float* pos, float* nrm, float* feedb
     h->last_out_set = h->set;
     h->have_last_out = true;
     return (h->count_valid && h->count_cached > cap) ? HPMC_ERR_CAPACITY : HPMC_OK;
+}
+
+// Waits for the stream; the last build's total and status.  The build's last
+// reduction has written them to mapped host memory (the copy this replaces cost
+// about 10 us a call).
+bool read_count(HPMCHistoPyramid* h, Ctrl* c) {
+    if (cudaStreamSynchronize(h->stream) != cudaSuccess) return false;
+    if (!h->host) return cudaMemcpy(c, h->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost) == cudaSuccess;
+    const volatile hpmc::HostCount* s = h->host;
+    c->total = s->total;
+    c->status = s->status;
+    return true;
 }
 
 // A build may overlap the previous extraction (Volume::overlap) when it
@@ -515,8 +533,7 @@ GLuint HPMCacquireNumberOfVertices(HPMCHistoPyramid* h) {
     if (!h->built) return 0;               // init.cpp:146-147: count starts at zero
     if (!h->count_valid) {
         Ctrl c;
-        if (cudaStreamSynchronize(h->stream) != cudaSuccess ||
-            cudaMemcpy(&c, h->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost) != cudaSuccess) {
+        if (!read_count(h, &c)) {
             set_error(h, HPMC_ERR_CUDA, true);
             return 0;
         }
@@ -524,6 +541,7 @@ GLuint HPMCacquireNumberOfVertices(HPMCHistoPyramid* h) {
             // reported once: the next build starts from a clean status word
             // (the handle may be un-broken by a setter that does not taint)
             cudaMemsetAsync(&h->d_ctrl->status, 0, sizeof(unsigned int), h->stream);
+            if (h->host) h->host->status = 0;
         }
         if (c.status & hpmc::kStatusTimeout) {
             set_error(h, HPMC_ERR_TIMEOUT, true);
@@ -690,12 +708,11 @@ int HPMCextractVerticesToBuffers(HPMCTraversalHandle* th, float* pos, float* nrm
     if (st != HPMC_OK && st != HPMC_ERR_CAPACITY) return st;
     if (n_written) {
         Ctrl c;
-        if (cudaStreamSynchronize(th->h->stream) != cudaSuccess ||
-            cudaMemcpy(&c, th->h->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost) != cudaSuccess) {
+        if (!read_count(th->h, &c)) {
             set_error(th->h, HPMC_ERR_CUDA, true);
             return HPMC_ERR_CUDA;
         }
-        *n_written = c.written;
+        *n_written = (uint32_t)std::min<unsigned long long>(c.total, cap);  // what the traversal writes
         if (c.total > cap) st = HPMC_ERR_CAPACITY;
     }
     return st;
@@ -769,7 +786,7 @@ int HPMCextractVerticesIndexed(HPMCTraversalHandle* th, float* positions, float*
     M.table_vals = reinterpret_cast<uint32_t*>(m + o_tvals);
     M.tile_sums = reinterpret_cast<uint32_t*>(m + o_tiles);
     M.meta = reinterpret_cast<uint16_t*>(m + o_meta);
-    M.unique = reinterpret_cast<unsigned long long*>(m + o_unique);
+    M.unique = h->host ? &h->host->unique : reinterpret_cast<unsigned int*>(m + o_unique);
     M.table_mask = (uint32_t)(tsize - 1);
     M.pos = reinterpret_cast<float4*>(positions);
     M.nrm = reinterpret_cast<float4*>(normals);
@@ -778,9 +795,11 @@ int HPMCextractVerticesIndexed(HPMCTraversalHandle* th, float* positions, float*
     M.icap = index_capacity;
     const int grid = h->constants->num_sms * 8;
     cudaError_t e = hpmc::launch_mesh(h->V, M, h->normal_mode, traverse_grid(h), grid, h->stream);
-    unsigned long long unique = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&unique, M.unique, sizeof unique, cudaMemcpyDeviceToHost, h->stream);
+    unsigned int unique = 0;
+    if (e == cudaSuccess && !h->host)
+        e = cudaMemcpyAsync(&unique, M.unique, sizeof unique, cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    if (e == cudaSuccess && h->host) unique = *static_cast<volatile unsigned int*>(&h->host->unique);
     if (e != cudaSuccess) {
         cudaGetLastError();
         set_error(h, HPMC_ERR_CUDA, true);
@@ -880,6 +899,7 @@ int HPMCgetDeviceStatus(HPMCHistoPyramid* h, unsigned int* status) {
     *status = c.status;
     const unsigned int zero = 0;
     cudaMemcpy(&h->d_ctrl->status, &zero, sizeof zero, cudaMemcpyHostToDevice);
+    if (h->host) h->host->status = 0;
     return HPMC_OK;
 }
 

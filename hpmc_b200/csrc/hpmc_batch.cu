@@ -86,6 +86,10 @@ struct HPMCBatch {
     } key{};
     bool have_graph = false;
     cudaStream_t last_stream = nullptr;
+    // status and offsets of the last extraction in mapped host memory (null for
+    // very many volumes, whose offsets are copied when they are asked for)
+    unsigned long long* host = nullptr;
+    bool extracted = false;
 };
 
 namespace {
@@ -100,6 +104,8 @@ void release(HPMCBatch* b) {
     b->capture_stream = nullptr;
     cudaFree(b->d_base);
     b->d_base = nullptr;
+    cudaFreeHost(b->host);
+    b->host = nullptr;
 }
 
 // Column depth of every volume and the brick prefix arrays.
@@ -158,6 +164,7 @@ BatchDev device_view(const HPMCBatch* b, size_t cap) {
     B.vbase = b->d_vbase;
     B.chunk_start = b->d_chunk_start;
     B.ctrl = b->d_bctrl;
+    B.host = b->host;
     B.capacity = cap;
     B.nvol = b->nvol;
     B.rounds = b->rounds;
@@ -238,6 +245,7 @@ int run(HPMCBatch* b, float* pos, float* nrm, size_t cap, cudaStream_t st) {
         return HPMC_ERR_CUDA;
     }
     b->last_stream = st;
+    b->extracted = true;
     return HPMC_OK;
 }
 
@@ -362,6 +370,13 @@ int HPMCcreateBatch(HPMCConstants* c, const HPMCBatchVolume* volumes, int count,
         delete b;
         return HPMC_ERR_CUDA;
     }
+    constexpr int kMaxHostOffsets = 4096;
+    if (count <= kMaxHostOffsets &&
+        cudaHostAlloc(reinterpret_cast<void**>(&b->host), sizeof(unsigned long long) * (count + 3), cudaHostAllocMapped) !=
+            cudaSuccess) {
+        cudaGetLastError();
+        b->host = nullptr;
+    }
     b->d_bctrl = reinterpret_cast<BatchCtrl*>(b->d_base + o_bctrl);
     b->d_ctrls = reinterpret_cast<Ctrl*>(b->d_base + o_ctrls);
     uint32_t* d_levels = reinterpret_cast<uint32_t*>(b->d_base + o_levels);
@@ -462,6 +477,17 @@ int HPMCbatchGetOffsets(HPMCBatch* b, unsigned long long* host_offsets) {
     if (!valid(b)) return HPMC_ERR_INVALID_HANDLE;
     if (!host_offsets) return HPMC_ERR_INVALID_VALUE;
     BatchCtrl bc;
+    if (b->host && b->extracted) {
+        if (cudaStreamSynchronize(b->last_stream) != cudaSuccess) {
+            cudaGetLastError();
+            return HPMC_ERR_CUDA;
+        }
+        if (*static_cast<volatile unsigned long long*>(b->host) == 0ull) {
+            std::memcpy(host_offsets, b->host + 2, sizeof(unsigned long long) * (b->nvol + 1));
+            return HPMC_OK;
+        }
+    }
+    // status bits to report and clear, or no copy on the host
     if (cudaStreamSynchronize(b->last_stream) != cudaSuccess ||
         cudaMemcpy(host_offsets, b->d_vbase, sizeof(unsigned long long) * (b->nvol + 1), cudaMemcpyDeviceToHost) !=
             cudaSuccess ||

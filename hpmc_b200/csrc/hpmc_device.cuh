@@ -82,6 +82,14 @@ struct Ctrl {
     unsigned int pad[3];
 };
 
+// What a build leaves for the host, in mapped host memory: written by the last
+// reduction and read after a synchronisation, without a copy.
+struct HostCount {
+    unsigned long long total;
+    unsigned int status;      // the status bits at that point
+    unsigned int unique;      // indexed output: distinct vertices of the last mesh
+};
+
 enum : unsigned int {
     kStatusOverflow = 1u,      // vertex count does not fit the level type
     kStatusCapacity = 2u,      // output buffer smaller than the vertex count
@@ -135,6 +143,7 @@ struct Volume {
     int slot_words;                    // kRowSlotWords (column layout) or kCodeSlotWords
     long long arena_slots;             // capacity of the arena
     Ctrl* ctrl;
+    HostCount* host;                   // may be null
     // optional capture of every cell's code, [cz][cy][cx] (inspection)
     uint8_t* codes_out;
     unsigned long long vertex_base;    // first output index of this volume (batched)

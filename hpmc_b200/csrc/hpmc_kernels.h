@@ -46,6 +46,7 @@ struct BatchDev {
     unsigned long long* vbase;     // nvol + 1: first output vertex of volume v (written by the reduction)
     uint32_t* chunk_start;         // nvol + 1: traversal work items before volume v (written by the reduction)
     BatchCtrl* ctrl;
+    unsigned long long* host;      // mapped host memory (may be null): status bits, unused, nvol + 1 offsets
     unsigned long long capacity;   // vertices the outputs can hold
     int nvol;
     int rounds;                    // traversal rounds of 32 vertices per work item
@@ -62,7 +63,7 @@ struct MeshIO {
     uint32_t* first;                 // count
     uint32_t* scan;                  // count
     uint32_t* tile_sums;             // count / 2048 + 1
-    unsigned long long* unique;      // 1: unique vertices
+    unsigned int* unique;            // 1: unique vertices (mapped host or device memory)
     float4* pos;                     // unique vertices (may be null)
     float4* nrm;
     unsigned long long vcap;

@@ -336,6 +336,15 @@ __device__ void reduce_tree(const Volume& V, uint32_t* buf0, uint32_t* buf1, int
     }
 }
 
+// The vertex count (one thread), after every status bit of the build.
+__device__ __forceinline__ void write_total(const Volume& V, uint32_t total) {
+    V.ctrl->total = total;
+    if (V.host) {
+        V.host->total = total;
+        V.host->status = __ldcg(&V.ctrl->status);
+    }
+}
+
 // One chunk of kReduceChunk level-j_in entries (chunk `chunk` of `nchunks`).
 // Returns true in the CTA that wrote the vertex count (level jtop reached).
 __device__ __forceinline__ bool reduce_chunk(const Volume& V, int j_in, int j_stop, long long chunk, unsigned int nchunks, uint32_t* buf0, uint32_t* buf1,
@@ -386,13 +395,11 @@ __device__ __forceinline__ bool reduce_chunk(const Volume& V, int j_in, int j_st
     }
     if (j < j_stop) {
         // levels remain above this chunk's top: the last CTA to finish continues
+        if (overflow) atomicOr(&V.ctrl->status, kStatusOverflow);
         __threadfence();
         if (threadIdx.x == 0) *s_last = (atomicAdd(&V.ctrl->reduce_done, 1u) == nchunks - 1);
         __syncthreads();
-        if (!*s_last) {
-            if (overflow) atomicOr(&V.ctrl->status, kStatusOverflow);
-            return false;
-        }
+        if (!*s_last) return false;
         __threadfence();
         const long long m = level_entries(V.size_l2, j);  // == nchunks entries, <= kReduceTop
         for (long long i = threadIdx.x; i < m; i += blockDim.x) buf0[i] = __ldcg(&V.levels[V.level_off[j] + i]);
@@ -401,7 +408,10 @@ __device__ __forceinline__ bool reduce_chunk(const Volume& V, int j_in, int j_st
         if (threadIdx.x == 0) V.ctrl->reduce_done = 0;
     }
     if (overflow) atomicOr(&V.ctrl->status, kStatusOverflow);
-    if (j == V.jtop && threadIdx.x == 0) V.ctrl->total = buf0[0];
+    if (j == V.jtop) {
+        __syncthreads();
+        if (threadIdx.x == 0) write_total(V, buf0[0]);
+    }
     return j == V.jtop;
 }
 
@@ -418,7 +428,7 @@ __global__ void __launch_bounds__(kThreads) reduce_levels(const __grid_constant_
 __global__ void copy_total(const __grid_constant__ Volume V) {
     wait_prior_grid();
     allow_next_grid();
-    if (threadIdx.x == 0) V.ctrl->total = V.levels[V.level_off[V.jtop]];
+    if (threadIdx.x == 0) write_total(V, V.levels[V.level_off[V.jtop]]);
 }
 
 // ---------------------------------------------------------------------------
@@ -495,13 +505,14 @@ __device__ void batch_scan(const BatchDev& B) {
     __shared__ uint32_t s_w32[kWarps];
     const uint32_t VW = 32u * (uint32_t)B.rounds;
     unsigned long long carry = 0;
-    uint32_t ccarry = 0;
+    uint32_t ccarry = 0, status = 0;
     for (int base = 0; base < B.nvol; base += kThreads) {
         const int v = base + (int)threadIdx.x;
         unsigned long long tot = 0;
         if (v < B.nvol) {
             const Ctrl* c = B.vols[v].ctrl;
             tot = __ldcg(&c->total);
+            status |= __ldcg(&c->status);
         }
         unsigned long long sum64;
         const unsigned long long vb = carry + block_exclusive_scan<unsigned long long>(tot, s_w64, sum64);
@@ -512,12 +523,23 @@ __device__ void batch_scan(const BatchDev& B) {
         const uint32_t cs = ccarry + block_exclusive_scan<uint32_t>(items, s_w32, sum32);
         if (v < B.nvol) {
             B.vbase[v] = vb;
+            if (B.host) B.host[2 + v] = vb;
             B.chunk_start[v] = cs;
         }
         carry += sum64;
         ccarry += sum32;
     }
+    if (carry > B.capacity) status |= kStatusCapacity;
+    status = __reduce_or_sync(0xffffffffu, status);
+    if ((threadIdx.x & 31) == 0) s_w32[threadIdx.x >> 5] = status;
+    __syncthreads();
     if (threadIdx.x == 0) {
+        if (B.host) {
+            for (int w = 1; w < kWarps; w++) status |= s_w32[w];
+            status |= __ldcg(&B.ctrl->status);  // not reported yet
+            B.host[0] = status;
+            B.host[2 + B.nvol] = carry;
+        }
         B.vbase[B.nvol] = carry;
         B.chunk_start[B.nvol] = ccarry;
         B.ctrl->total = carry;

@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(kThreads) mesh_first(const unsigned long long*
 
 // One CTA: exclusive scan of the tile sums in place; total into *unique.
 __global__ void __launch_bounds__(kThreads) mesh_scan_tiles(uint32_t* tile_sums, uint32_t ntiles,
-                                                            unsigned long long* unique) {
+                                                            unsigned int* unique) {
     __shared__ uint32_t s_warp[kWarps];
     uint32_t carry = 0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

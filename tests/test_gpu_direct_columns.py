@@ -50,7 +50,7 @@ def test_batch_without_tensor_maps(hpmc, dtype):
     else:
         fields, isos = [rng.integers(100, 156, size=s).astype(np.uint8) for s in shapes], [[128.0] * 6, [120.0] * 6]
     b = hpmc.Batch([torch.from_numpy(f).cuda() for f in fields], isos[0])
-    pos = torch.empty((400_000, 4), device="cuda")
+    pos = torch.empty((2_000_000, 4), device="cuda")
     nrm = torch.empty_like(pos)
     for values in isos:
         b.set_iso_values(values)
