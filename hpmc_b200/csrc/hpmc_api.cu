@@ -89,7 +89,12 @@ struct HPMCHistoPyramid {
     int nsets = 0;
     int set = 0;                   // the set of the last build
     Ctrl* d_ctrl = nullptr;
-    hpmc::HostCount* host = nullptr;  // where builds leave their count (mapped host memory), or null
+    // where builds leave their count (mapped host memory), or null.  A build
+    // writes it when the count of the build before was read: the write holds up
+    // the end of the reduction by about 1 us, which a loop that never reads the
+    // count need not pay.
+    hpmc::HostCount* host = nullptr;
+    bool count_read = true, host_written = false;
     // the last extraction's outputs (byte ranges), stream and set: the next
     // build overlaps it only on the same stream, into the other set, and with
     // a field that is none of those outputs
@@ -240,7 +245,6 @@ bool setup(HPMCHistoPyramid* h) {
     V.arena = h->d_arena;
     V.arena_slots = slots;
     V.ctrl = h->d_ctrl;
-    V.host = h->host;
     h->set = 0;
     h->tainted = false;
     h->built = false;
@@ -297,12 +301,13 @@ int launch_extract(HPMCTraversalHandle* th, float* pos, float* nrm, float* feedb
     return (h->count_valid && h->count_cached > cap) ? HPMC_ERR_CAPACITY : HPMC_OK;
 }
 
-// Waits for the stream; the last build's total and status.  The build's last
-// reduction has written them to mapped host memory (the copy this replaces cost
-// about 10 us a call).
+// Waits for the stream; the last build's total and status.  In a loop that
+// reads them the build's last reduction has written them to mapped host memory
+// (the copy this replaces cost about 10 us a call).
 bool read_count(HPMCHistoPyramid* h, Ctrl* c) {
     if (cudaStreamSynchronize(h->stream) != cudaSuccess) return false;
-    if (!h->host) return cudaMemcpy(c, h->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost) == cudaSuccess;
+    h->count_read = true;
+    if (!h->host_written) return cudaMemcpy(c, h->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost) == cudaSuccess;
     const volatile hpmc::HostCount* s = h->host;
     c->total = s->total;
     c->status = s->status;
@@ -509,6 +514,9 @@ void HPMCbuildHistopyramid(HPMCHistoPyramid* h, GLfloat threshold) {
         V.arena = h->d_arena + (size_t)h->set * h->arena_cap;
     }
     V.overlap = may_overlap_extraction(h) ? 1 : 0;
+    V.host = h->count_read ? h->host : nullptr;
+    h->host_written = V.host != nullptr;
+    h->count_read = false;
     h->threshold = threshold;
     const int max_ctas = h->constants->num_sms * 16;
     cudaError_t e;

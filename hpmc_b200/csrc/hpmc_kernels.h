@@ -46,7 +46,7 @@ struct BatchDev {
     unsigned long long* vbase;     // nvol + 1: first output vertex of volume v (written by the reduction)
     uint32_t* chunk_start;         // nvol + 1: traversal work items before volume v (written by the reduction)
     BatchCtrl* ctrl;
-    unsigned long long* host;      // mapped host memory (may be null): status bits, unused, nvol + 1 offsets
+    unsigned long long* host;      // mapped host memory (may be null): any status bit set, unused, nvol + 1 offsets
     unsigned long long capacity;   // vertices the outputs can hold
     int nvol;
     int rounds;                    // traversal rounds of 32 vertices per work item

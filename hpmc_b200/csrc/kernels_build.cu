@@ -505,14 +505,13 @@ __device__ void batch_scan(const BatchDev& B) {
     __shared__ uint32_t s_w32[kWarps];
     const uint32_t VW = 32u * (uint32_t)B.rounds;
     unsigned long long carry = 0;
-    uint32_t ccarry = 0, status = 0;
+    uint32_t ccarry = 0;
     for (int base = 0; base < B.nvol; base += kThreads) {
         const int v = base + (int)threadIdx.x;
         unsigned long long tot = 0;
         if (v < B.nvol) {
             const Ctrl* c = B.vols[v].ctrl;
             tot = __ldcg(&c->total);
-            status |= __ldcg(&c->status);
         }
         unsigned long long sum64;
         const unsigned long long vb = carry + block_exclusive_scan<unsigned long long>(tot, s_w64, sum64);
@@ -523,23 +522,12 @@ __device__ void batch_scan(const BatchDev& B) {
         const uint32_t cs = ccarry + block_exclusive_scan<uint32_t>(items, s_w32, sum32);
         if (v < B.nvol) {
             B.vbase[v] = vb;
-            if (B.host) B.host[2 + v] = vb;
             B.chunk_start[v] = cs;
         }
         carry += sum64;
         ccarry += sum32;
     }
-    if (carry > B.capacity) status |= kStatusCapacity;
-    status = __reduce_or_sync(0xffffffffu, status);
-    if ((threadIdx.x & 31) == 0) s_w32[threadIdx.x >> 5] = status;
-    __syncthreads();
     if (threadIdx.x == 0) {
-        if (B.host) {
-            for (int w = 1; w < kWarps; w++) status |= s_w32[w];
-            status |= __ldcg(&B.ctrl->status);  // not reported yet
-            B.host[0] = status;
-            B.host[2 + B.nvol] = carry;
-        }
         B.vbase[B.nvol] = carry;
         B.chunk_start[B.nvol] = ccarry;
         B.ctrl->total = carry;

@@ -198,6 +198,18 @@ __global__ void __launch_bounds__(kThreads, kTraverseCtas) traverse_batch(const 
     TraverseSmem& S = *reinterpret_cast<TraverseSmem*>(s_traverse);
     load_base_tables(S);
     __syncthreads();
+    if (Bt.host && blockIdx.x == 0) {
+        // offsets and whether any status bit is set, for the host: from here the
+        // writes across PCIe overlap the traversal (from the reduction they
+        // would hold up its end by 2 us)
+        uint32_t status = threadIdx.x == 0 ? __ldcg(&Bt.ctrl->status) : 0u;
+        for (int v = (int)threadIdx.x; v <= Bt.nvol; v += kThreads) {
+            Bt.host[2 + v] = __ldcg(Bt.vbase + v);
+            if (v < Bt.nvol) status |= __ldcg(&Bt.vols[v].ctrl->status);
+        }
+        status = (uint32_t)__syncthreads_or((int)status);
+        if (threadIdx.x == 0) Bt.host[0] = status;
+    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t VW = 32u * (uint32_t)Bt.rounds;
     const uint32_t nitems = __ldcg(Bt.chunk_start + Bt.nvol);
