@@ -433,21 +433,25 @@ template <class P>
 __device__ __forceinline__ void walk_range(const Volume& V, const TraverseSmem& S, WarpArea& W, int lane, uint32_t v0,
                                            uint32_t v1, uint32_t N, P& p) {
     WarpBlock B;
-    descend(V, S, v0, B.b, B.base, B.count);
-    locate_block(V, B);
-    uint32_t queued = 0, pos = 0, visit = 0;
+    uint32_t queued = 0, pos = 0, visit = 0, next = v0;
+    bool found = false;  // B is the block of vertex `next`, and located
     // this lane's cell in a tile and the first cell of tile `lane`, x | y << 5
     const uint32_t in_tile = morton_tile_cell((uint32_t)lane);
     const uint32_t tile_at = morton_tile_x((uint32_t)lane) | ((uint32_t)morton_tile_y((uint32_t)lane) << 5);
     for (;;) {
-        const uint32_t next = B.base + B.count;
+        if (!found) {
+            descend(V, S, next, B.b, B.base, B.count);
+            locate_block(V, B);
+        }
+        next = B.base + B.count;
         const bool more = next < v1 && B.count != 0u;
         const uint32_t sib = more ? sibling_counts(V, lane, B.b) : 0u;
         load_block(V, W, lane, B);
         const uint32_t sm = __ballot_sync(0xffffffffu, sib != 0u);
-        const uint32_t ahead = (uint32_t)__ffs((int)sm);  // the next block is b + ahead (0: a descent finds it)
+        found = sm != 0u;
         WarpBlock N1 = B;
-        if (sm) {
+        if (found) {
+            const uint32_t ahead = (uint32_t)__ffs((int)sm);  // the next block is b + ahead
             N1.b += ahead;
             N1.base = next;
             N1.count = __shfl_sync(0xffffffffu, sib, (int)ahead - 1);
@@ -459,7 +463,8 @@ __device__ __forceinline__ void walk_range(const Volume& V, const TraverseSmem& 
         // (nothing is queued before the first block)
         if (!queued && tiles) pos = B.base + __shfl_sync(0xffffffffu, B.tstart, __ffs((int)tiles) - 1);
         uint32_t listed = 0;
-        while (tiles || listed) {
+        // the last block also empties the queue
+        while (tiles || listed || (!more && queued)) {
             while (listed < kWindowCells && tiles) {
                 const int t = __ffs((int)tiles) - 1;
                 tiles &= tiles - 1u;
@@ -490,25 +495,20 @@ __device__ __forceinline__ void walk_range(const Volume& V, const TraverseSmem& 
             W.list[lane] = (uint16_t)later;  // the cells past these 32 move up
             listed -= n;
             queued += n;
-            if (queued >= kWindowCells) {
+            if (queued >= kWindowCells || (!more && !tiles && !listed)) {
                 const uint2 rest = W.cell[kWindowCells + lane];
-                process_window(V, S, W, lane, kWindowCells, pos, v0, v1, N, p);
+                const uint32_t m = min(queued, (uint32_t)kWindowCells);
+                process_window(V, S, W, lane, m, pos, v0, v1, N, p);
                 __syncwarp();
                 W.cell[lane] = rest;
-                queued -= kWindowCells;
+                queued -= m;
             }
             __syncwarp();
         }
         if (!more) break;
-        if (sm) {
-            B = N1;
-        } else {
-            descend(V, S, next, B.b, B.base, B.count);
-            locate_block(V, B);
-        }
+        if (found) B = N1;
         visit = (visit + 1u) & 63u;
     }
-    if (queued) process_window(V, S, W, lane, queued, pos, v0, v1, N, p);
     __syncwarp();
 }
 
@@ -630,7 +630,7 @@ struct ExtractVertices {
             float4* pos = O.pos + o0 + G.lane;
             float4* nrm = O.nrm + o0 + G.lane;
             const bool p = O.pos != nullptr, q = O.nrm != nullptr;
-#pragma unroll 2
+#pragma unroll 1
             for (uint32_t i = (uint32_t)G.lane; i < n; i += 32, pos += 32, nrm += 32) {
                 const float2* d = &W.data[0][W.slot[i]];
                 const float2 d0 = d[0], d1 = d[kWindowEdges], d2 = d[2 * kWindowEdges];
