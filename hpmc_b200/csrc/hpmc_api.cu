@@ -762,15 +762,18 @@ int HPMCextractVerticesIndexed(HPMCTraversalHandle* th, float* positions, float*
     if (h->V.ftype == hpmc::kFieldUser) return HPMC_ERR_UNSUPPORTED;  // its kernels live in the caller's code
     const GLuint n = HPMCacquireNumberOfVertices(h);  // sizes the scratch (host sync)
     if (n == 0 && h->status != HPMC_OK) return h->status;
-    // scratch: keys | table keys | first | scan | table vals | tile sums | meta | unique count
+    // scratch: keys | table keys, table vals | vertex | first | place | bits | scan | tile sums | meta | unique count.
+    // More table slots than soup vertices: an edge has at least one of them, and
+    // about six, so the table is at most a third full off the grid's boundary.
     size_t tsize = 1;
-    while (tsize < 2 * (size_t)n + 2) tsize <<= 1;
-    const size_t tiles = (size_t)n / 2048 + 2;
+    while (tsize < (size_t)n + 2) tsize <<= 1;
+    const size_t words = ((size_t)n + 31) / 32;
     auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
-    const size_t o_keys = 0, o_tkeys = up(o_keys + 8 * (size_t)n), o_first = up(o_tkeys + 8 * tsize),
-                 o_scan = up(o_first + 4 * (size_t)n), o_tvals = up(o_scan + 4 * (size_t)n),
-                 o_tiles = up(o_tvals + 4 * tsize), o_meta = up(o_tiles + 4 * tiles),
-                 o_unique = up(o_meta + 2 * (size_t)n), bytes = o_unique + 256;
+    const size_t o_keys = 0, o_tkeys = up(o_keys + 8 * (size_t)n), o_vertex = up(o_tkeys + 12 * tsize),
+                 o_first = up(o_vertex + 4 * (size_t)n), o_place = up(o_first + 4 * (size_t)n),
+                 o_bits = up(o_place + 4 * (size_t)n), o_scan = up(o_bits + 4 * words), o_tiles = up(o_scan + 4 * words),
+                 o_meta = up(o_tiles + 4 * ((size_t)n / 65536 + 2)), o_unique = up(o_meta + 2 * (size_t)n),
+                 bytes = o_unique + 256;
     if (!th->mesh_mem || th->mesh_cap < bytes) {
         if (th->mesh_mem) {
             cudaStreamSynchronize(h->stream);
@@ -789,9 +792,12 @@ int HPMCextractVerticesIndexed(HPMCTraversalHandle* th, float* positions, float*
     M.count = n;
     M.keys = reinterpret_cast<unsigned long long*>(m + o_keys);
     M.table_keys = reinterpret_cast<unsigned long long*>(m + o_tkeys);
+    M.vertex = reinterpret_cast<uint32_t*>(m + o_vertex);
     M.first = reinterpret_cast<uint32_t*>(m + o_first);
+    M.place = reinterpret_cast<uint32_t*>(m + o_place);
+    M.table_vals = reinterpret_cast<uint32_t*>(m + o_tkeys + 8 * tsize);
+    M.bits = reinterpret_cast<uint32_t*>(m + o_bits);
     M.scan = reinterpret_cast<uint32_t*>(m + o_scan);
-    M.table_vals = reinterpret_cast<uint32_t*>(m + o_tvals);
     M.tile_sums = reinterpret_cast<uint32_t*>(m + o_tiles);
     M.meta = reinterpret_cast<uint16_t*>(m + o_meta);
     M.unique = h->host ? &h->host->unique : reinterpret_cast<unsigned int*>(m + o_unique);

@@ -79,7 +79,9 @@ struct Ctrl {
     unsigned int col_next;       // column classifier's work queue: next column to claim
     unsigned int col_done;       // column classifier CTAs finished (the last one resets the queue)
     unsigned int extracting;     // nonzero while an extraction of this pyramid runs (traverse_kernel)
-    unsigned int pad[3];
+    unsigned int mesh_edges;     // indexed output: edges listed so far (the last kernel resets it)
+    unsigned int mesh_done;      // indexed output: scan CTAs finished (the last one resets it)
+    unsigned int pad;
 };
 
 // What a build leaves for the host, in mapped host memory: written by the last

@@ -52,17 +52,22 @@ struct BatchDev {
     int rounds;                    // traversal rounds of 32 vertices per work item
 };
 
-// Indexed-mesh extraction: scratch and outputs (device).
+// Indexed-mesh extraction: scratch and outputs (device).  An "edge" below is a
+// distinct edge of one group of cells of the traversal (at most `count` in all);
+// its number of listed edges is Ctrl::mesh_edges.
 struct MeshIO {
     uint32_t count;                  // soup vertices (the vertex count of the build)
-    unsigned long long* keys;        // count: edge key per soup vertex
-    uint16_t* meta;                  // count: case | vertex-in-cell << 8
-    unsigned long long* table_keys;  // table_mask + 1 (>= 2 count, power of two)
-    uint32_t* table_vals;
+    uint32_t* vertex;                // count: edge of each soup vertex
+    uint16_t* meta;                  // count: case | vertex-in-cell << 8 (binary fields only)
+    unsigned long long* keys;        // per edge: mesh_key
+    uint32_t* first;                 // per edge: its smallest soup index in the group
+    uint32_t* place;                 // per edge: table slot, then number of its vertex
+    unsigned long long* table_keys;  // table_mask + 1 (> count, power of two)
+    uint32_t* table_vals;            // right behind table_keys
     uint32_t table_mask;
-    uint32_t* first;                 // count
-    uint32_t* scan;                  // count
-    uint32_t* tile_sums;             // count / 2048 + 1
+    uint32_t* bits;                  // (count + 31) / 32: soup vertices that are the first on their edge
+    uint32_t* scan;                  // per word of bits: set bits before it in its tile
+    uint32_t* tile_sums;             // count / 65536 + 2
     unsigned int* unique;            // 1: unique vertices (mapped host or device memory)
     float4* pos;                     // unique vertices (may be null)
     float4* nrm;

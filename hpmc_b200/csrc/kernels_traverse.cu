@@ -245,62 +245,90 @@ __global__ void __launch_bounds__(kThreads, kTraverseCtas) traverse_batch(const 
 // welding keeps one vertex per edge, numbered in order of first occurrence
 // in the soup, and an index per soup vertex (three per triangle, the soup's
 // triangle order).
-//   mesh_keys   traversal without geometry: the edge key of every soup vertex
-//               (and its case / vertex-in-cell, for binary-field normals);
-//   mesh_insert open-addressing table key -> smallest soup index (atomicCAS
-//               on the key, atomicMin on the index);
-//   mesh_first  per soup vertex: that smallest index, and a flag "first";
-//   mesh_scan_* exclusive scan of the flags = unique vertex numbers;
-//   mesh_emit   indices, and the geometry of each unique vertex computed once
-//               from its edge (bit-identical to the soup vertex's).
-__device__ __forceinline__ unsigned long long edge_key(const Volume& V, const int a[3], int axis) {
-    return ((((unsigned long long)a[2] * (unsigned long long)V.lattice[1]) + (unsigned long long)a[1]) *
-                (unsigned long long)V.lattice[0] + (unsigned long long)a[0]) * 3ull + (unsigned long long)axis;
+//   mesh_edges    traversal without geometry: lists every group's distinct
+//                 edges with their first soup vertex in the group, and per soup
+//                 vertex its edge; clears the table;
+//   mesh_insert   open-addressing table key -> smallest soup index (atomicCAS
+//                 on the key, atomicMin on the index), an edge's slot kept;
+//   mesh_mark     one bit per soup vertex that is the first on its edge;
+//   mesh_scan     exclusive scan of the bits = unique vertex numbers;
+//   mesh_vertices per edge its number, and for the first one the geometry
+//                 (bit-identical to the soup vertex's);
+//   mesh_indices  per soup vertex its edge's number.
+// The table sees a group's distinct edges, 0.4 per soup vertex, and is probed
+// once for each (every soup vertex inserted and looked up: 99 us of kernels at
+// 192^3 with 0.9 M soup vertices).  Bound by launches and atomics in L2.
+__device__ __forceinline__ unsigned long long mesh_key(const int a[3], int axis) {
+    return (unsigned long long)a[0] | ((unsigned long long)a[1] << 14) | ((unsigned long long)a[2] << 28) |
+           ((unsigned long long)axis << 42);
 }
 
-struct EdgeKeys {
-    unsigned long long* keys;
-    uint16_t* meta;
+constexpr unsigned long long kEmptyKey = ~0ull;
+
+struct MeshEdges {
+    const MeshIO& M;
+    unsigned int* count;
+    bool meta;
 
     __device__ __forceinline__ void run(const CellGroup& G) {
-        unsigned long long* slots = reinterpret_cast<unsigned long long*>(G.W.data[0]);
-        G.edges([&](uint32_t slot, const EdgeAt& E) { slots[slot] = edge_key(G.V, E.a, E.axis); });
+        unsigned long long* key = reinterpret_cast<unsigned long long*>(G.W.data[0]);
+        uint32_t* first = reinterpret_cast<uint32_t*>(G.W.data[1]);
+        uint32_t j0 = 0;
+        if (G.lane == 0) j0 = atomicAdd(count, G.nedges);
+        j0 = __shfl_sync(0xffffffffu, j0, 0);
+        G.edges([&](uint32_t slot, const EdgeAt& E) {
+            key[slot] = mesh_key(E.a, E.axis);
+            first[slot] = 0xffffffffu;
+        });
         const uint32_t n = G.last - G.first;
-        uint32_t c0 = (uint32_t)__ffs((int)G.lanes) - 2u;
+        for (uint32_t i = (uint32_t)G.lane; i < n; i += 32) {
+            const uint32_t slot = G.W.slot[i];
+            atomicMin(&first[slot], G.first + i);
+            M.vertex[G.first + i] = j0 + slot;
+        }
+        if (meta) {
+            uint32_t c0 = (uint32_t)__ffs((int)G.lanes) - 2u;
 #pragma unroll 1
-        for (uint32_t i0 = 0; i0 < n; i0 += 32) {
-            const uint32_t i = i0 + (uint32_t)G.lane, starts = G.starts(i0);
-            const int c = (int)((c0 + (uint32_t)__popc(starts & (0xffffffffu >> (31 - G.lane)))) & 31u);
-            c0 += (uint32_t)__popc(starts);
-            const uint32_t code = __shfl_sync(0xffffffffu, G.code, c);
-            const uint32_t k = (G.first + i - __shfl_sync(0xffffffffu, G.start, c)) & 15u;
-            if (i >= n) continue;
-            keys[G.first + i] = slots[G.W.slot[i]];
-            meta[G.first + i] = (uint16_t)(code | (k << 8));
+            for (uint32_t i0 = 0; i0 < n; i0 += 32) {
+                const uint32_t i = i0 + (uint32_t)G.lane, starts = G.starts(i0);
+                const int c = (int)((c0 + (uint32_t)__popc(starts & (0xffffffffu >> (31 - G.lane)))) & 31u);
+                c0 += (uint32_t)__popc(starts);
+                const uint32_t code = __shfl_sync(0xffffffffu, G.code, c);
+                const uint32_t k = (G.first + i - __shfl_sync(0xffffffffu, G.start, c)) & 15u;
+                if (i < n) M.meta[G.first + i] = (uint16_t)(code | (k << 8));
+            }
+        }
+        __syncwarp();
+        for (uint32_t i = (uint32_t)G.lane; i < G.nedges; i += 32) {
+            M.keys[j0 + i] = key[i];
+            M.first[j0 + i] = first[i];
         }
         __syncwarp();
     }
 };
 
-__global__ void __launch_bounds__(kThreads, kTraverseCtas) mesh_keys(const __grid_constant__ Volume V,
-                                                                     unsigned long long* keys, uint16_t* meta,
-                                                                     uint32_t count) {
+__global__ void __launch_bounds__(kThreads, kTraverseCtas) mesh_edges(const __grid_constant__ Volume V,
+                                                                      const __grid_constant__ MeshIO M) {
     extern __shared__ __align__(16) uint8_t s_traverse[];
     TraverseSmem& S = *reinterpret_cast<TraverseSmem*>(s_traverse);
     load_tables(V, S);
+    allow_next_grid();
+    const uint32_t t0 = blockIdx.x * kThreads + threadIdx.x, nt = gridDim.x * kThreads;
+    uint4* table = reinterpret_cast<uint4*>(M.table_keys);  // keys and, behind them, vals: a multiple of 16 bytes
+    const size_t quads = 3 * ((size_t)M.table_mask + 1) / 4;
+    for (size_t i = t0; i < quads; i += nt) table[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+    for (uint32_t i = t0; i < (M.count + 31u) / 32u; i += nt) M.bits[i] = 0u;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned long long total = V.ctrl->total;
-    const uint32_t N = (uint32_t)(total < count ? total : count);
+    const uint32_t N = (uint32_t)(total < M.count ? total : M.count);
     const uint32_t VW = 32u * item_rounds(N, gridDim.x);
     const uint32_t nchunks = (N + VW - 1) / VW;
     set_volume(V, S.warp[warp], lane);
-    EdgeKeys p{keys, meta};
+    MeshEdges p{M, &V.ctrl->mesh_edges, V.binary != 0};
     for (uint32_t chunk = next_chunk(V, lane); chunk < nchunks; chunk = next_chunk(V, lane))
         walk_range(V, S, S.warp[warp], lane, chunk * VW, min(N, (chunk + 1u) * VW), N, p);
     finish_queue(V);
 }
-
-constexpr unsigned long long kEmptyKey = ~0ull;
 
 __device__ __forceinline__ uint32_t key_hash(unsigned long long k) {
     k ^= k >> 33;
@@ -309,189 +337,164 @@ __device__ __forceinline__ uint32_t key_hash(unsigned long long k) {
     return (uint32_t)k;
 }
 
-__global__ void mesh_insert(const unsigned long long* keys, uint32_t n, unsigned long long* tkeys, uint32_t* tvals,
-                            uint32_t mask, unsigned int* status) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const unsigned long long key = keys[i];
-        uint32_t h = key_hash(key) & mask;
-        bool done = false;
-        for (uint32_t probe = 0; probe <= mask; probe++) {  // the table has >= 2n slots: ends long before
-            const unsigned long long prev = atomicCAS(&tkeys[h], kEmptyKey, key);
+__global__ void __launch_bounds__(kThreads) mesh_insert(const __grid_constant__ MeshIO M, Ctrl* ctrl) {
+    wait_prior_grid();
+    allow_next_grid();
+    const uint32_t n = __ldcg(&ctrl->mesh_edges);
+    for (uint32_t j = blockIdx.x * kThreads + threadIdx.x; j < n; j += gridDim.x * kThreads) {
+        const unsigned long long key = M.keys[j];
+        uint32_t h = key_hash(key) & M.table_mask, place = 0xffffffffu;
+        for (uint32_t probe = 0; probe <= M.table_mask; probe++) {  // the table has more slots than keys
+            const unsigned long long prev = atomicCAS(&M.table_keys[h], kEmptyKey, key);
             if (prev == kEmptyKey || prev == key) {
-                atomicMin(&tvals[h], i);
-                done = true;
+                atomicMin(&M.table_vals[h], M.first[j]);
+                place = h;
                 break;
             }
-            h = (h + 1u) & mask;
+            h = (h + 1u) & M.table_mask;
         }
-        if (!done) atomicOr(status, kStatusCapacity);
+        M.place[j] = place;
+        if (place == 0xffffffffu) atomicOr(&ctrl->status, kStatusCapacity);
     }
 }
 
-__device__ __forceinline__ uint32_t table_find(const unsigned long long* tkeys, const uint32_t* tvals, uint32_t mask,
-                                               unsigned long long key) {
-    uint32_t h = key_hash(key) & mask;
-    for (uint32_t probe = 0; probe <= mask; probe++) {
-        const unsigned long long k = tkeys[h];
-        if (k == key) return tvals[h];
-        if (k == kEmptyKey) break;
-        h = (h + 1u) & mask;
+__global__ void __launch_bounds__(kThreads) mesh_mark(const __grid_constant__ MeshIO M, Ctrl* ctrl) {
+    wait_prior_grid();
+    allow_next_grid();
+    const uint32_t n = __ldcg(&ctrl->mesh_edges);
+    for (uint32_t j = blockIdx.x * kThreads + threadIdx.x; j < n; j += gridDim.x * kThreads) {
+        const uint32_t h = M.place[j], f = M.first[j];
+        if (h <= M.table_mask && M.table_vals[h] == f) atomicOr(&M.bits[f >> 5], 1u << (f & 31u));
     }
-    return 0xffffffffu;
 }
 
-constexpr int kScanItems = 8;                        // per thread
-constexpr uint32_t kScanTile = kThreads * kScanItems; // per CTA
+constexpr int kScanItems = 8;                          // words of bits per thread
+constexpr uint32_t kScanTile = kThreads * kScanItems;  // per CTA
 
-__global__ void __launch_bounds__(kThreads) mesh_first(const unsigned long long* keys, uint32_t n,
-                                                       const unsigned long long* tkeys, const uint32_t* tvals,
-                                                       uint32_t mask, uint32_t* first, uint32_t* scan,
-                                                       uint32_t* tile_sums) {
-    // first[i] = smallest soup index of i's edge; scan[i] = exclusive count of
-    // firsts within the tile; tile_sums[tile] = firsts in the tile
+// scan[w] = bits set before word w in its tile; the last CTA turns the tiles'
+// sums into their exclusive scan and writes the number of unique vertices.
+__global__ void __launch_bounds__(kThreads) mesh_scan(const __grid_constant__ MeshIO M, Ctrl* ctrl) {
     __shared__ uint32_t s_warp[kWarps];
+    __shared__ int s_last;
+    wait_prior_grid();
+    allow_next_grid();
+    const uint32_t words = (M.count + 31u) / 32u;
     const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    uint32_t f[kScanItems], sum = 0;
-#pragma unroll
-    for (int j = 0; j < kScanItems; j++) {
-        const uint32_t i = base + j;
-        uint32_t fi = 0u;
-        if (i < n) {
-            const uint32_t m = table_find(tkeys, tvals, mask, keys[i]);
-            first[i] = m;
-            fi = (m == i) ? 1u : 0u;
-        }
-        f[j] = fi;
-        sum += fi;
-    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t inc = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += y;
-    }
-    if (lane == 31) s_warp[warp] = inc;
-    __syncthreads();
-    uint32_t off = 0, tot = 0;
-#pragma unroll
-    for (int w = 0; w < kWarps; w++) {
-        if (w < warp) off += s_warp[w];
-        tot += s_warp[w];
-    }
-    uint32_t run = off + inc - sum;
-#pragma unroll
-    for (int j = 0; j < kScanItems; j++) {
-        const uint32_t i = base + j;
-        if (i < n) scan[i] = run;
-        run += f[j];
-    }
-    if (threadIdx.x == 0) tile_sums[blockIdx.x] = tot;
-}
-
-// One CTA: exclusive scan of the tile sums in place; total into *unique.
-__global__ void __launch_bounds__(kThreads) mesh_scan_tiles(uint32_t* tile_sums, uint32_t ntiles,
-                                                            unsigned int* unique) {
-    __shared__ uint32_t s_warp[kWarps];
-    uint32_t carry = 0;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (uint32_t b = 0; b < ntiles; b += kThreads) {
-        const uint32_t i = b + threadIdx.x;
-        const uint32_t x = i < ntiles ? tile_sums[i] : 0u;
-        uint32_t inc = x;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += y;
-        }
+    auto block_scan = [&](uint32_t x, uint32_t& total) {  // exclusive
+        const uint32_t inc = warp_inclusive_scan(x, lane);
         if (lane == 31) s_warp[warp] = inc;
         __syncthreads();
-        uint32_t off = 0, tot = 0;
+        uint32_t off = 0;
+        total = 0;
 #pragma unroll
         for (int w = 0; w < kWarps; w++) {
             if (w < warp) off += s_warp[w];
-            tot += s_warp[w];
+            total += s_warp[w];
         }
-        if (i < ntiles) tile_sums[i] = carry + off + inc - x;
-        carry += tot;
         __syncthreads();
+        return off + inc - x;
+    };
+    uint32_t f[kScanItems], sum = 0, total;
+#pragma unroll
+    for (int j = 0; j < kScanItems; j++) {
+        f[j] = base + j < words ? (uint32_t)__popc(__ldcg(&M.bits[base + j])) : 0u;
+        sum += f[j];
     }
-    if (threadIdx.x == 0) *unique = carry;
+    uint32_t run = block_scan(sum, total);
+#pragma unroll
+    for (int j = 0; j < kScanItems; j++) {
+        if (base + j < words) M.scan[base + j] = run;
+        run += f[j];
+    }
+    if (threadIdx.x == 0) {
+        M.tile_sums[blockIdx.x] = total;
+        __threadfence();
+        s_last = atomicAdd(&ctrl->mesh_done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    uint32_t carry = 0;
+    for (uint32_t b = 0; b < gridDim.x; b += kThreads) {
+        const uint32_t i = b + threadIdx.x;
+        const uint32_t off = block_scan(i < gridDim.x ? __ldcg(&M.tile_sums[i]) : 0u, total);
+        if (i < gridDim.x) M.tile_sums[i] = carry + off;
+        carry += total;
+    }
+    if (threadIdx.x == 0) {
+        *M.unique = carry;
+        ctrl->mesh_done = 0;
+    }
 }
 
 template <int FT, int MODE>
-__global__ void __launch_bounds__(kThreads) mesh_emit(const __grid_constant__ Volume V, const unsigned long long* keys,
-                                                      const uint16_t* meta, uint32_t n, const uint32_t* first,
-                                                      const uint32_t* scan, const uint32_t* tile_sums, float4* pos,
-                                                      float4* nrm, unsigned long long vcap, uint32_t* indices,
-                                                      unsigned long long icap) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t j = first[i];
-        if (j >= n) continue;  // not found: the insert reported it
-        const uint32_t u = scan[j] + tile_sums[j / kScanTile];
-        if (indices && i < icap) indices[i] = u;
-        if (j != i || u >= vcap) continue;
-        // the unique vertex: geometry from its edge
-        const unsigned long long key = keys[i];
-        const int axis = (int)(key % 3ull);
-        unsigned long long r = key / 3ull;
-        int a[3];
-        a[0] = (int)(r % (unsigned long long)V.lattice[0]);
-        r /= (unsigned long long)V.lattice[0];
-        a[1] = (int)(r % (unsigned long long)V.lattice[1]);
-        a[2] = (int)(r / (unsigned long long)V.lattice[1]);
-        const uint16_t m = meta[i];
-        const int code = m & 0xff, k = (m >> 8) & 15;
+__global__ void __launch_bounds__(kThreads) mesh_vertices(const __grid_constant__ Volume V,
+                                                          const __grid_constant__ MeshIO M) {
+    wait_prior_grid();
+    allow_next_grid();
+    const uint32_t n = __ldcg(&V.ctrl->mesh_edges);
+    for (uint32_t j = blockIdx.x * kThreads + threadIdx.x; j < n; j += gridDim.x * kThreads) {
+        const uint32_t h = M.place[j];
+        if (h > M.table_mask) continue;  // not inserted: reported there
+        const uint32_t f = M.table_vals[h], word = f >> 5;
+        const uint32_t u = M.tile_sums[word / kScanTile] + M.scan[word] +
+                           (uint32_t)__popc(M.bits[word] & ((1u << (f & 31u)) - 1u));
+        M.place[j] = u;
+        if (M.first[j] != f || u >= M.vcap) continue;
+        const unsigned long long key = M.keys[j];
         float p[3], nn[3], t;
-        edge_vertex<FT, MODE>(V, edge_at(V, a[0], a[1], a[2], (uint32_t)axis << 3), p, nn, t);
+        edge_vertex<FT, MODE>(V, edge_at(V, (int)(key & 0x3fffu), (int)((key >> 14) & 0x3fffu), (int)((key >> 28) & 0x3fffu),
+                                         (uint32_t)(key >> 42) << 3), p, nn, t);
         if (MODE == kModeBinary) {
+            const uint16_t m = M.meta[f];
 #pragma unroll
-            for (int c = 0; c < 3; c++) nn[c] = g_binary_normals[3 * (16 * code + k) + c] * V.scale[c];
+            for (int c = 0; c < 3; c++) nn[c] = g_binary_normals[3 * (16 * (m & 0xff) + ((m >> 8) & 15)) + c] * V.scale[c];
         }
-        if (pos) pos[u] = make_float4(p[0], p[1], p[2], 1.0f);
-        if (nrm) nrm[u] = make_float4(nn[0], nn[1], nn[2], 0.0f);
+        if (M.pos) M.pos[u] = make_float4(p[0], p[1], p[2], 1.0f);
+        if (M.nrm) M.nrm[u] = make_float4(nn[0], nn[1], nn[2], 0.0f);
     }
+}
+
+__global__ void __launch_bounds__(kThreads) mesh_indices(const __grid_constant__ MeshIO M, Ctrl* ctrl) {
+    wait_prior_grid();
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->mesh_edges = 0;
+    if (!M.indices) return;
+    const uint32_t n = (uint32_t)(M.icap < M.count ? M.icap : M.count);
+    for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads)
+        M.indices[i] = M.place[M.vertex[i]];
+}
+
+template <int FT>
+static cudaError_t launch_mesh_vertices(const Volume& V, const MeshIO& M, int mode, int grid, cudaStream_t st) {
+    return mode == kModeBinary    ? launch_dependent(mesh_vertices<FT, kModeBinary>, grid, kThreads, 0, st, V, M)
+           : mode == kModeCentral ? launch_dependent(mesh_vertices<FT, kModeCentral>, grid, kThreads, 0, st, V, M)
+                                  : launch_dependent(mesh_vertices<FT, kModeForward>, grid, kThreads, 0, st, V, M);
 }
 
 cudaError_t launch_mesh(const Volume& V, const MeshIO& M, int normal_mode, int traverse_grid, int grid,
                         cudaStream_t st) {
-    const uint32_t n = M.count;
     static std::atomic<uint64_t> devices{0};
-    cudaError_t e = allow_traverse_smem(mesh_keys, kTraverseSmem, devices);
-    if (e != cudaSuccess) return e;
-    mesh_keys<<<traverse_grid, kThreads, kTraverseSmem, st>>>(V, M.keys, M.meta, n);
-    e = cudaGetLastError();
-    if (e != cudaSuccess || n == 0) return e;
-    if ((e = cudaMemsetAsync(M.table_keys, 0xff, sizeof(unsigned long long) * (M.table_mask + 1ull), st)) !=
-            cudaSuccess ||
-        (e = cudaMemsetAsync(M.table_vals, 0xff, sizeof(uint32_t) * (M.table_mask + 1ull), st)) != cudaSuccess)
-        return e;
-    mesh_insert<<<grid, kThreads, 0, st>>>(M.keys, n, M.table_keys, M.table_vals, M.table_mask, &V.ctrl->status);
-    const uint32_t ntiles = (n + kScanTile - 1) / kScanTile;
-    mesh_first<<<ntiles, kThreads, 0, st>>>(M.keys, n, M.table_keys, M.table_vals, M.table_mask, M.first, M.scan,
-                                            M.tile_sums);
-    mesh_scan_tiles<<<1, kThreads, 0, st>>>(M.tile_sums, ntiles, M.unique);
+    cudaError_t e = allow_traverse_smem(mesh_edges, kTraverseSmem, devices);
+    if (e != cudaSuccess || M.count == 0) return e;
     const int mode = V.binary ? kModeBinary : (normal_mode == kNormalsCentral ? kModeCentral : kModeForward);
-#define HPMC_MESH_EMIT(FT_, MODE_)                                                                             \
-    mesh_emit<FT_, MODE_><<<grid, kThreads, 0, st>>>(V, M.keys, M.meta, n, M.first, M.scan, M.tile_sums, M.pos,  \
-                                                     M.nrm, M.vcap, M.indices, M.icap)
-#define HPMC_MESH_CASE(FT_)                                                                                    \
-    case FT_:                                                                                                  \
-        if (mode == kModeBinary) HPMC_MESH_EMIT(FT_, kModeBinary);                                             \
-        else if (mode == kModeCentral) HPMC_MESH_EMIT(FT_, kModeCentral);                                      \
-        else HPMC_MESH_EMIT(FT_, kModeForward);                                                                \
-        break;
-    switch (V.ftype) {
-        HPMC_MESH_CASE(kFieldF32)
-        HPMC_MESH_CASE(kFieldU8)
-        HPMC_MESH_CASE(kFieldUNorm8)
-        HPMC_MESH_CASE(kFieldFunctor)
-        HPMC_MESH_CASE(kFieldF32X4)
-        default: return cudaErrorInvalidValue;
+    const unsigned int tiles = ((M.count + 31u) / 32u + kScanTile - 1) / kScanTile;
+    e = launch_dependent(mesh_edges, traverse_grid, kThreads, kTraverseSmem, st, V, M);
+    if (e == cudaSuccess) e = launch_dependent(mesh_insert, grid, kThreads, 0, st, M, V.ctrl);
+    if (e == cudaSuccess) e = launch_dependent(mesh_mark, grid, kThreads, 0, st, M, V.ctrl);
+    if (e == cudaSuccess) e = launch_dependent(mesh_scan, tiles, kThreads, 0, st, M, V.ctrl);
+    if (e == cudaSuccess) {
+        switch (V.ftype) {
+            case kFieldF32: e = launch_mesh_vertices<kFieldF32>(V, M, mode, grid, st); break;
+            case kFieldU8: e = launch_mesh_vertices<kFieldU8>(V, M, mode, grid, st); break;
+            case kFieldUNorm8: e = launch_mesh_vertices<kFieldUNorm8>(V, M, mode, grid, st); break;
+            case kFieldFunctor: e = launch_mesh_vertices<kFieldFunctor>(V, M, mode, grid, st); break;
+            case kFieldF32X4: e = launch_mesh_vertices<kFieldF32X4>(V, M, mode, grid, st); break;
+            default: return cudaErrorInvalidValue;
+        }
     }
-#undef HPMC_MESH_CASE
-#undef HPMC_MESH_EMIT
-    return cudaGetLastError();
+    if (e == cudaSuccess) e = launch_dependent(mesh_indices, grid, kThreads, 0, st, M, V.ctrl);
+    return e;
 }
 
 // ---------------------------------------------------------------------------

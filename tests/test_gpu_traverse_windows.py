@@ -71,3 +71,32 @@ def test_plain_extraction(hpmc, oracle, name, normals):
     np.testing.assert_array_equal(p[:n], pos[:n])
     p, q = run(n, (False, True))
     np.testing.assert_array_equal(q[:n], nrm[:n])
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+@pytest.mark.parametrize("binary", [False, True])
+def test_welded_equals_soup(hpmc, name, binary):
+    """The indexed output over the same fields: indices name first occurrences
+    in order, and a unique vertex is its first soup vertex, bit for bit."""
+    import torch
+
+    field = _field(*CASES[name])
+    hp = hpmc.HistoPyramid(hpmc.default_constants())
+    hp.set_field_device(torch.from_numpy(field).cuda())
+    if binary:
+        hp.set_field_as_binary()
+    for _ in range(2):  # the scratch is reused
+        hp.build(0.0)
+        n = hp.acquire_number_of_vertices()
+        th = hpmc.TraversalHandle(hp)
+        pos, nrm, p, q = (torch.full((n, 4), float("nan"), device="cuda") for _ in range(4))
+        idx = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+        th.extract_to(pos, nrm, n)
+        unique, ni = th.extract_indexed(p, q, idx)
+        assert ni == n
+        idx = idx.cpu().numpy()
+        new = np.maximum.accumulate(np.concatenate(([-1], idx[:-1]))) < idx  # first occurrences, numbered in order
+        assert new.sum() == unique and (idx[new] == np.arange(unique)).all()
+        np.testing.assert_array_equal(p[:unique].cpu().numpy(), pos.cpu().numpy()[new])
+        np.testing.assert_array_equal(q[:unique].cpu().numpy(), nrm.cpu().numpy()[new])
+        np.testing.assert_array_equal(p.cpu().numpy()[idx], pos.cpu().numpy())  # a position per edge
