@@ -6,7 +6,7 @@
 //
 // Device memory of a batch (one allocation):
 //   batch control block | per-volume control blocks | descriptors |
-//   tensor maps | brick, reduce-chunk and work-item prefix arrays |
+//   tensor maps | bricks, reduce-chunk and work-item prefix arrays |
 //   output offsets | dense levels of every volume | block arenas
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -57,16 +57,18 @@ struct HPMCBatch {
     std::vector<Volume> hv;            // descriptors (device pointers filled in)
     std::vector<uint8_t> column;       // volume uses the TMA column classifier
     std::vector<CUtensorMap> tmaps;
-    std::vector<uint32_t> brick_start, direct_start, reduce_start;
-    unsigned int bricks = 0, direct_bricks = 0, reduce_chunks = 0;
+    std::vector<uint2> bricks, direct_bricks;  // BatchDev's, for the current column depth
+    std::vector<uint32_t> reduce_start;
+    unsigned int reduce_chunks = 0;
+    size_t max_bricks = 0, max_direct = 0;     // at the smallest column depth
     // device
     unsigned char* d_base = nullptr;
     BatchCtrl* d_bctrl = nullptr;
     Ctrl* d_ctrls = nullptr;
     Volume* d_vols = nullptr;
     CUtensorMap* d_tmaps = nullptr;
-    uint32_t* d_brick_start = nullptr;
-    uint32_t* d_direct_start = nullptr;
+    uint2* d_bricks = nullptr;
+    uint2* d_direct_bricks = nullptr;
     uint32_t* d_reduce_start = nullptr;
     uint32_t* d_chunk_start = nullptr;
     unsigned long long* d_vbase = nullptr;
@@ -74,7 +76,9 @@ struct HPMCBatch {
     int column_slices = 0;
     int traverse_ctas_per_sm = 0;
     int rounds = hpmc::kTraverseRounds;
-    bool upload = true;  // descriptors / prefix arrays changed since the last upload
+    bool upload = true;         // descriptors changed since the last upload
+    bool upload_bricks = true;  // the bricks did
+    int stall_volume = -1, stall_box = -1;
     // captured graph and what it was captured for
     cudaStream_t capture_stream = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -82,7 +86,7 @@ struct HPMCBatch {
         float* pos;
         float* nrm;
         size_t cap;
-        int mode, zc, ctas, rounds;
+        int mode, zc, ctas, rounds, stall_volume, stall_box;
     } key{};
     bool have_graph = false;
     cudaStream_t last_stream = nullptr;
@@ -108,7 +112,7 @@ void release(HPMCBatch* b) {
     b->host = nullptr;
 }
 
-// Column depth of every volume and the brick prefix arrays.
+// Column depth of every volume and the bricks.
 void apply_column_slices(HPMCBatch* b) {
     int zc = b->column_slices;
     if (zc == 0) {
@@ -125,21 +129,26 @@ void apply_column_slices(HPMCBatch* b) {
             }
         }
     }
-    uint32_t acc = 0, direct = 0;
+    b->bricks.clear();
+    b->direct_bricks.clear();
     for (int v = 0; v < b->nvol; v++) {
         Volume& V = b->hv[v];
         V.column_slices = zc;
-        b->brick_start[v] = acc;
-        b->direct_start[v] = direct;
-        const uint32_t columns = (uint32_t)(V.nfx * V.nfy * ((V.cells[2] + zc - 1) / zc));
-        if (b->column[v]) acc += columns;
-        else direct += V.column_layout ? columns : (uint32_t)V.nblocks;
+        const int nz = (V.cells[2] + zc - 1) / zc;
+        if (!b->column[v]) {
+            const long long n = V.column_layout ? (long long)V.nfx * V.nfy * nz : V.nblocks;
+            for (long long i = 0; i < n; i++) b->direct_bricks.push_back(make_uint2((uint32_t)v, (uint32_t)i));
+            continue;
+        }
+        for (int z = 0; z < nz; z++)
+            for (int y = 0; y < V.nfy; y++)
+                for (int x = 0; x < V.nfx; x++) {
+                    const uint32_t slices = (uint32_t)std::min(zc, V.cells[2] - z * zc);
+                    b->bricks.push_back(make_uint2((uint32_t)v | (slices << 20),
+                                                   (uint32_t)x | ((uint32_t)y << 9) | ((uint32_t)z << 18)));
+                }
     }
-    b->brick_start[b->nvol] = acc;
-    b->direct_start[b->nvol] = direct;
-    b->bricks = acc;
-    b->direct_bricks = direct;
-    b->upload = true;
+    b->upload = b->upload_bricks = true;
 }
 
 int max_traverse_ctas() {
@@ -158,8 +167,11 @@ BatchDev device_view(const HPMCBatch* b, size_t cap) {
     BatchDev B{};
     B.vols = b->d_vols;
     B.tmaps = b->d_tmaps;
-    B.brick_start = b->d_brick_start;
-    B.direct_start = b->d_direct_start;
+    B.bricks = b->d_bricks;
+    B.direct_bricks = b->d_direct_bricks;
+    B.column_slices = b->hv[0].column_slices;
+    B.stall_volume = b->stall_volume;
+    B.stall_box = b->stall_box;
     B.reduce_start = b->d_reduce_start;
     B.vbase = b->d_vbase;
     B.chunk_start = b->d_chunk_start;
@@ -174,8 +186,8 @@ BatchDev device_view(const HPMCBatch* b, size_t cap) {
 // The launches of one batched extraction, on `st` (captured into the graph).
 cudaError_t issue(HPMCBatch* b, float* pos, float* nrm, size_t cap, int traverse_grid, cudaStream_t st) {
     const BatchDev B = device_view(b, cap);
-    cudaError_t e = hpmc::launch_classify_batch_direct(B, b->ftype, b->direct_bricks, st);
-    if (e == cudaSuccess) e = hpmc::launch_classify_batch(B, b->ftype, b->bricks, st);
+    cudaError_t e = hpmc::launch_classify_batch_direct(B, b->ftype, (unsigned int)b->direct_bricks.size(), st);
+    if (e == cudaSuccess) e = hpmc::launch_classify_batch(B, b->ftype, (unsigned int)b->bricks.size(), st);
     if (e == cudaSuccess) e = hpmc::launch_reduce_batch(B, b->reduce_chunks, st);
     if (e == cudaSuccess) {
         hpmc::TraverseOut O{};
@@ -194,19 +206,25 @@ int upload(HPMCBatch* b, cudaStream_t st) {
             cudaSuccess ||
         cudaMemcpyAsync(b->d_tmaps, b->tmaps.data(), sizeof(CUtensorMap) * b->nvol, cudaMemcpyHostToDevice, st) !=
             cudaSuccess ||
-        cudaMemcpyAsync(b->d_brick_start, b->brick_start.data(), n1, cudaMemcpyHostToDevice, st) != cudaSuccess ||
-        cudaMemcpyAsync(b->d_direct_start, b->direct_start.data(), n1, cudaMemcpyHostToDevice, st) != cudaSuccess ||
         cudaMemcpyAsync(b->d_reduce_start, b->reduce_start.data(), n1, cudaMemcpyHostToDevice, st) != cudaSuccess) {
         cudaGetLastError();
         return HPMC_ERR_CUDA;
     }
-    b->upload = false;
+    if (b->upload_bricks &&
+        (cudaMemcpyAsync(b->d_bricks, b->bricks.data(), sizeof(uint2) * b->bricks.size(), cudaMemcpyHostToDevice, st) !=
+             cudaSuccess ||
+         cudaMemcpyAsync(b->d_direct_bricks, b->direct_bricks.data(), sizeof(uint2) * b->direct_bricks.size(),
+                         cudaMemcpyHostToDevice, st) != cudaSuccess)) {
+        cudaGetLastError();
+        return HPMC_ERR_CUDA;
+    }
+    b->upload = b->upload_bricks = false;
     return HPMC_OK;
 }
 
 int ensure_graph(HPMCBatch* b, float* pos, float* nrm, size_t cap) {
     const HPMCBatch::Key k{pos, nrm, cap, b->normal_mode, b->hv.empty() ? 0 : b->hv[0].column_slices,
-                           effective_ctas(b), b->rounds};
+                           effective_ctas(b), b->rounds, b->stall_volume, b->stall_box};
     if (b->have_graph && std::memcmp(&k, &b->key, sizeof k) == 0) return HPMC_OK;
     if (b->exec) cudaGraphExecDestroy(b->exec);
     b->exec = nullptr;
@@ -271,8 +289,6 @@ int HPMCcreateBatch(HPMCConstants* c, const HPMCBatchVolume* volumes, int count,
     b->hv.assign(count, Volume{});
     b->column.assign(count, 0);
     b->tmaps.assign(count, CUtensorMap{});
-    b->brick_start.assign(count + 1, 0);
-    b->direct_start.assign(count + 1, 0);
     b->reduce_start.assign(count + 1, 0);
 
     // per-volume layouts and sizes
@@ -321,6 +337,10 @@ int HPMCcreateBatch(HPMCConstants* c, const HPMCBatchVolume* volumes, int count,
         V.u8_thr = hpmc::host::u8_threshold(V.ftype, s.iso);
         if (V.column_layout && ((uintptr_t)s.field % 16 == 0) && rp % 16 == 0 && sp % 16 == 0)
             b->column[v] = hpmc::host::encode_column_map(&b->tmaps[v], s.field, stype, lattice, rp, sp) ? 1 : 0;
+        const size_t columns = (size_t)V.nfx * V.nfy *
+                               ((V.cells[2] + hpmc::kColumnSliceChoices[3] - 1) / hpmc::kColumnSliceChoices[3]);
+        if (b->column[v]) b->max_bricks += columns;
+        else b->max_direct += V.column_layout ? columns : (size_t)V.nblocks;
         lev_off[v] = lev_total;
         lev_total += lev;  // a multiple of 4 entries: every volume's levels stay 16-byte aligned
         V.arena_slots = slots;
@@ -347,9 +367,9 @@ int HPMCcreateBatch(HPMCConstants* c, const HPMCBatchVolume* volumes, int count,
     const size_t o_tmaps = off;
     off = align_up(off + sizeof(CUtensorMap) * count, 256);
     const size_t o_brick = off;
-    off = align_up(off + sizeof(uint32_t) * (count + 1), 256);
+    off = align_up(off + sizeof(uint2) * b->max_bricks, 256);
     const size_t o_direct = off;
-    off = align_up(off + sizeof(uint32_t) * (count + 1), 256);
+    off = align_up(off + sizeof(uint2) * b->max_direct, 256);
     const size_t o_red = off;
     off = align_up(off + sizeof(uint32_t) * (count + 1), 256);
     const size_t o_chunk = off;
@@ -382,8 +402,8 @@ int HPMCcreateBatch(HPMCConstants* c, const HPMCBatchVolume* volumes, int count,
     uint32_t* d_levels = reinterpret_cast<uint32_t*>(b->d_base + o_levels);
     b->d_vols = reinterpret_cast<Volume*>(b->d_base + o_vols);
     b->d_tmaps = reinterpret_cast<CUtensorMap*>(b->d_base + o_tmaps);
-    b->d_brick_start = reinterpret_cast<uint32_t*>(b->d_base + o_brick);
-    b->d_direct_start = reinterpret_cast<uint32_t*>(b->d_base + o_direct);
+    b->d_bricks = reinterpret_cast<uint2*>(b->d_base + o_brick);
+    b->d_direct_bricks = reinterpret_cast<uint2*>(b->d_base + o_direct);
     b->d_reduce_start = reinterpret_cast<uint32_t*>(b->d_base + o_red);
     b->d_chunk_start = reinterpret_cast<uint32_t*>(b->d_base + o_chunk);
     b->d_vbase = reinterpret_cast<unsigned long long*>(b->d_base + o_vbase);
@@ -451,8 +471,9 @@ int HPMCbatchGetTuning(HPMCBatch* b, int out[3]) {
 int HPMCbatchSetTestStall(HPMCBatch* b, int volume, int box, unsigned int wait_limit_us) {
     if (!valid(b)) return HPMC_ERR_INVALID_HANDLE;
     if (volume < 0 || volume >= b->nvol) return HPMC_ERR_INVALID_VALUE;
+    b->stall_volume = box >= 0 ? volume : -1;
+    b->stall_box = box >= 0 ? box : -1;
     for (int v = 0; v < b->nvol; v++) {
-        b->hv[v].stall_box = (v == volume && box >= 0) ? box : -1;
         b->hv[v].wait_limit_ns = wait_limit_us ? 1000ull * wait_limit_us : hpmc::kWaitLimitNs;
     }
     b->upload = true;

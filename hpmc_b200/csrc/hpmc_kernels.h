@@ -40,8 +40,9 @@ struct BatchCtrl {
 struct BatchDev {
     const Volume* vols;            // per-volume descriptors (top_cached = 0)
     const CUtensorMap* tmaps;      // per-volume column tensor maps (64-byte aligned)
-    const uint32_t* brick_start;   // nvol + 1: column bricks before volume v (volumes with a tensor map)
-    const uint32_t* direct_start;  // nvol + 1: columns or blocks before volume v (the other volumes)
+    const uint2* bricks;           // column bricks of the volumes with a tensor map: volume | slices << 20,
+                                   // fx | fy << 9 | (first slice / column_slices) << 18
+    const uint2* direct_bricks;    // of the other volumes: volume, column or block
     const uint32_t* reduce_start;  // nvol + 1: reduction chunks before volume v
     unsigned long long* vbase;     // nvol + 1: first output vertex of volume v (written by the reduction)
     uint32_t* chunk_start;         // nvol + 1: traversal work items before volume v (written by the reduction)
@@ -49,6 +50,8 @@ struct BatchDev {
     unsigned long long* host;      // mapped host memory (may be null): any status bit set, unused, nvol + 1 offsets
     unsigned long long capacity;   // vertices the outputs can hold
     int nvol;
+    int column_slices;             // of every volume
+    int stall_volume, stall_box;   // test hook (Volume::stall_box), -1: off
     int rounds;                    // traversal rounds of 32 vertices per work item
 };
 
