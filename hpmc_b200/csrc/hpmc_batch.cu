@@ -75,6 +75,7 @@ struct HPMCBatch {
     // tuning (column_slices 0 = automatic)
     int column_slices = 0;
     int traverse_ctas_per_sm = 0;
+    int default_rounds = hpmc::kTraverseRounds;
     int rounds = hpmc::kTraverseRounds;
     bool upload = true;         // descriptors changed since the last upload
     bool upload_bricks = true;  // the bricks did
@@ -350,6 +351,9 @@ int HPMCcreateBatch(HPMCConstants* c, const HPMCBatchVolume* volumes, int count,
         const long long n5 = hpmc::level_entries(V.size_l2, hpmc::kBlockLevel);
         chunks += (uint32_t)std::max(1ll, (n5 + 1023) / 1024);
     }
+    long long cells = 0;
+    for (const Volume& V : b->hv) cells += (long long)V.cells[0] * V.cells[1] * V.cells[2];
+    if (cells >= hpmc::kLargeBatchCells) b->rounds = b->default_rounds = hpmc::kLargeBatchRounds;
     b->reduce_start[count] = chunks;
     b->reduce_chunks = chunks;
 
@@ -454,7 +458,7 @@ int HPMCbatchSetTuning(HPMCBatch* b, int column_slices, int traverse_ctas_per_sm
     if (!zc_ok || traverse_ctas_per_sm < 0 || rounds < 0 || rounds > 64) return HPMC_ERR_INVALID_VALUE;
     b->column_slices = column_slices;
     b->traverse_ctas_per_sm = traverse_ctas_per_sm;
-    b->rounds = rounds ? rounds : hpmc::kTraverseRounds;
+    b->rounds = rounds ? rounds : b->default_rounds;
     apply_column_slices(b);
     return HPMC_OK;
 }
@@ -562,7 +566,7 @@ int HPMCbatchAutotune(HPMCBatch* b, float* positions, float* normals, size_t cap
     }
     const int maxc = max_traverse_ctas();
     float best = 1e30f;
-    int bz = 0, bc = 0, br = hpmc::kTraverseRounds;
+    int bz = 0, bc = 0, br = b->default_rounds;
     int status = HPMC_OK;
     for (int zc : hpmc::kColumnSliceChoices) {
         for (int ctas : kTraverseCtaChoices) {

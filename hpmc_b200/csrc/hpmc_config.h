@@ -29,10 +29,14 @@ constexpr int kTopCacheEntries = 344;
 constexpr int kTraverseCtas = 3;
 // Rounds of 32 vertices a warp of the single-volume traversal takes at least.
 constexpr int kMinRounds = 4;
-// Vertices per warp work item (R rounds of 32) of the batched traversal (its
-// default; the autotuner chooses) and of the host's grid sizing; the
-// single-volume traversal gives each warp one contiguous range instead.
+// Vertices per warp work item (R rounds of 32) of the batched traversal, until
+// tuned: longer items save descents and part windows, but leave warps without
+// work in a small batch.  8, 16, 32 rounds: 64 volumes of 84 M cells 447, 394,
+// 384 us; 24 of 8 M cells 95, 95, 103.  The single-volume traversal gives each
+// warp one contiguous range instead.
 constexpr int kTraverseRounds = 8;
+constexpr int kLargeBatchRounds = 16;
+constexpr long long kLargeBatchCells = 16ll << 20;
 
 // Bounded waits: an mbarrier poll gives up after this long (a TMA box lands
 // in microseconds; only a fault in the copy path gets near it).
