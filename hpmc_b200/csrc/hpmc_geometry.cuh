@@ -58,6 +58,20 @@ __device__ __forceinline__ float ff_lerp(FF A, FF B, FF t) {
     return r.hi + r.lo;
 }
 
+// A + t (B - A) with A = a - b, B = c - d for floats and t float-float, rounded
+// once: every rounding error of a difference, the product and the sum is found
+// exactly and added up with the low parts, so what is lost is of second order,
+// as with ff_lerp (35 operations instead of 62).
+__device__ __forceinline__ float lerp_of_diffs(float a, float b, float c, float d, FF t) {
+    const FF A = two_sum(a, -b), B = two_sum(c, -d);
+    const FF D = two_sum(B.hi, -A.hi);
+    const float dlo = D.lo + (B.lo - A.lo);
+    const float p = t.hi * D.hi;
+    const float pe = fmaf(t.hi, D.hi, -p);
+    const FF s = two_sum(A.hi, p);
+    return s.hi + (s.lo + (pe + (fmaf(t.hi, dlo, t.lo * D.hi) + A.lo)));
+}
+
 // Integer lattice index -> float without the conversion pipe (0 <= v < 2^23).
 __device__ __forceinline__ float index_to_float(int v) { return __int_as_float(0x4B000000 | v) - 8388608.0f; }
 
@@ -258,10 +272,8 @@ __device__ __forceinline__ void edge_vertex(const Volume& V, const EdgeAt& E, fl
             const FF tf = ff_ratio_of_diffs(F.va, iso, F.va, F.vb);
 #pragma unroll
             for (int i = 0; i < 3; i++) {
-                if (MODE == kGeomForward)
-                    r[i] = ff_lerp(two_sum(iso, -hiA[i]), two_sum(iso, -hiB[i]), tf);
-                else
-                    r[i] = ff_lerp(two_sum(hiA[i], -loA[i]), two_sum(hiB[i], -loB[i]), tf);
+                r[i] = MODE == kGeomForward ? lerp_of_diffs(iso, hiA[i], iso, hiB[i], tf)
+                                            : lerp_of_diffs(hiA[i], loA[i], hiB[i], loB[i], tf);
             }
             t = tf.hi + tf.lo;
         }
