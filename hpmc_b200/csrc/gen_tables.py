@@ -15,7 +15,13 @@ The derivations below restate ``hpmc/src/constants.cpp``:
                          exactly as the reference's host code does, then the
                          traversal's ``2*fract(v)-1`` (shadergen.cpp:507-510).
 
-Usage: python gen_tables.py <hpmc source tree> <output header>
+Where no HPMC tree is at hand, the same three arrays follow from the golden
+fixtures (``tests/golden/*.npz``), whose extractions list code, vertex and edge
+of every case and positions on every edge; ``--fixtures`` writes them as a
+``tables.cpp`` for the oracle's build.
+
+Usage: python gen_tables.py <hpmc source tree or fixtures directory> <output header>
+       python gen_tables.py --fixtures <fixtures directory> <output tables.cpp>
 """
 from __future__ import annotations
 
@@ -57,6 +63,43 @@ def read_reference_tables(hpmc_src: str):
     if tri.size != 256 * 16 or edge.size != 12 * 4 or mid.size != 12 * 3:
         raise ValueError("unexpected table sizes in tables.cpp")
     return tri.reshape(256, 16), edge.reshape(12, 4), mid.reshape(12, 3)
+
+
+def read_fixture_tables(golden: str):
+    """The arrays of read_reference_tables from the golden fixtures."""
+    tri = np.full((256, 16), -1, np.int64)
+    edge = np.full((12, 4), -1, np.float32)
+    code_edges = np.full((256, 16), -1, np.int64)
+    for name in sorted(f for f in os.listdir(golden) if f.endswith(".npz")):
+        d = np.load(os.path.join(golden, name))
+        code_edges[d["code"], d["k"]] = d["edge"]
+        if name != "normal_grid.npz":
+            continue
+        # the cell-relative position of a crossing: 0 or 1 on two axes, t on the edge's own
+        at = d["pos_fwd"] * np.array(d["codes"].shape[::-1]) - d["cell"]
+        inner = (d["t_fwd"] > 0.05) & (d["t_fwd"] < 0.95)
+        for e, p in zip(d["edge"][inner], at[inner]):
+            axis = int(np.argmax(np.abs(p - np.round(p))))
+            p = np.round(p)
+            p[axis] = 0
+            edge[e] = (*p, axis)
+    if (edge < 0).any() or (code_edges[1:255, 0] < 0).any():
+        raise ValueError(f"the fixtures in {golden} do not cover every case")
+    for j in range(256):
+        tri[j] = code_edges[remap(j)]
+    mid = edge[:, :3] + 0.5 * (edge[:, 3:] == np.arange(3))
+    return tri, edge, mid.astype(np.float32)
+
+
+def write_tables_cpp(out_path: str, tri, edge, mid) -> None:
+    def array(kind, name, a):
+        rows = ",\n".join("{" + ", ".join(repr(v) for v in row) + "}" for row in a.tolist())
+        return f"{kind} {name}[{a.shape[0]}][{a.shape[1]}] = {{\n{rows}}};\n"
+
+    os.makedirs(os.path.dirname(os.path.abspath(out_path)), exist_ok=True)
+    with open(out_path, "w") as f:
+        f.write(array("int", "HPMC_triangle_table", tri) + array("float", "HPMC_edge_table", edge)
+                + array("float", "HPMC_midpoint_table", mid))
 
 
 def remap(c: int) -> int:
@@ -151,11 +194,14 @@ def emit(out_path: str, tri, edge, mid) -> None:
 
 
 def main(argv):
+    if len(argv) == 4 and argv[1] == "--fixtures":
+        write_tables_cpp(argv[3], *read_fixture_tables(argv[2]))
+        return 0
     if len(argv) != 3:
         print(__doc__)
         return 2
-    tri, edge, mid = read_reference_tables(argv[1])
-    emit(argv[2], tri, edge, mid)
+    from_tree = os.path.exists(os.path.join(argv[1], "hpmc", "src", "tables.cpp"))
+    emit(argv[2], *(read_reference_tables if from_tree else read_fixture_tables)(argv[1]))
     return 0
 
 
