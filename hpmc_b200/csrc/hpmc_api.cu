@@ -95,6 +95,10 @@ struct HPMCHistoPyramid {
     // count need not pay.
     hpmc::HostCount* host = nullptr;
     bool count_read = true, host_written = false;
+    // the last build's stream; whether a build was ever captured into a graph,
+    // whose replays may run on any stream and after other builds
+    cudaStream_t build_stream = nullptr;
+    bool captured = false;
     // the last extraction's outputs (byte ranges), stream and set: the next
     // build overlaps it only on the same stream, into the other set, and with
     // a field that is none of those outputs
@@ -303,11 +307,14 @@ int launch_extract(HPMCTraversalHandle* th, float* pos, float* nrm, float* feedb
 
 // Waits for the stream; the last build's total and status.  In a loop that
 // reads them the build's last reduction has written them to mapped host memory
-// (the copy this replaces cost about 10 us a call).
+// (the copy this replaces cost about 10 us a call).  After a build on another
+// stream or in a captured graph, the copy, which also waits for the default
+// stream's work and reads what ran last.
 bool read_count(HPMCHistoPyramid* h, Ctrl* c) {
     if (cudaStreamSynchronize(h->stream) != cudaSuccess) return false;
     h->count_read = true;
-    if (!h->host_written) return cudaMemcpy(c, h->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost) == cudaSuccess;
+    if (!h->host_written || h->build_stream != h->stream)
+        return cudaMemcpy(c, h->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost) == cudaSuccess;
     const volatile hpmc::HostCount* s = h->host;
     c->total = s->total;
     c->status = s->status;
@@ -514,7 +521,14 @@ void HPMCbuildHistopyramid(HPMCHistoPyramid* h, GLfloat threshold) {
         V.arena = h->d_arena + (size_t)h->set * h->arena_cap;
     }
     V.overlap = may_overlap_extraction(h) ? 1 : 0;
-    V.host = h->count_read ? h->host : nullptr;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (!h->captured &&
+        (cudaStreamIsCapturing(h->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone)) {
+        cudaGetLastError();
+        h->captured = true;
+    }
+    V.host = h->count_read && !h->captured ? h->host : nullptr;
+    h->build_stream = h->stream;
     h->host_written = V.host != nullptr;
     h->count_read = false;
     h->threshold = threshold;

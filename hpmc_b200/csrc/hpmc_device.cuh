@@ -17,10 +17,11 @@
 //   * below block level nothing is stored densely: each block with a non-zero
 //     count gets an "arena" slot.  Column layout (every block inside one slice
 //     tile): the block's 33x33 sample bits (below the iso-value or not) of its
-//     lower and upper layer, 288 bytes, from which a traversal warp derives
-//     active cells, MC codes and crossed edges.  Otherwise: the block's 1024 MC
-//     codes in Morton order and the active mask of each of its 32-cell Morton
-//     tiles.  Levels 0..4 of the reference are thus implied: the traversal warp
+//     lower and upper layer and the vertex counts of its 32-cell Morton tiles,
+//     352 bytes, from which a traversal warp derives active cells, MC codes and
+//     crossed edges.  Otherwise: the block's 1024 MC codes in Morton order and
+//     the active masks and vertex counts of its 32-cell Morton tiles, 1,216
+//     bytes.  Levels 0..4 of the reference are thus implied: the traversal warp
 //     counts the vertices of the active cells in Morton (= vertex) order.
 //     Cells of empty blocks are all inside or all outside and are not needed.
 #pragma once
