@@ -12,7 +12,6 @@
 // of the tables in its own device module.
 #pragma once
 #include <cuda_runtime.h>
-#include <atomic>
 #include <cstdint>
 
 #include "hpmc_device.cuh"
@@ -88,6 +87,9 @@ constexpr size_t kTraverseSmem = sizeof(TraverseSmem);
 // Batched: a volume descriptor per warp follows.
 static_assert(sizeof(TraverseSmem) % 16 == 0 && kVolumeHead % 8 == 0, "descriptors are copied in 8-byte words");
 constexpr size_t kBatchSmem = sizeof(TraverseSmem) + kWarps * kVolumeHead;
+// Dynamic shared memory without an opt-in per kernel, device and context; the
+// adjoint has 6 KB of its own.
+static_assert(kBatchSmem <= 48 * 1024 && kTraverseSmem + 6 * 1024 <= 48 * 1024, "at most 48 KB");
 
 // The block a warp is working in: its vertices base .. base + count - 1, its
 // key-space origin and, for the column layout, the lattice cell of its first
@@ -572,19 +574,6 @@ __device__ __forceinline__ void finish_queue_batch(const BatchDev& Bt) {
     }
 }
 
-// Opts kernel K into kTraverseSmem bytes of dynamic shared memory, once per device.
-template <class K>
-inline cudaError_t allow_traverse_smem(K* kernel, size_t bytes, std::atomic<uint64_t>& devices) {
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    const uint64_t bit = 1ull << (dev & 63);
-    if (dev < 64 && (devices.load(std::memory_order_relaxed) & bit)) return cudaSuccess;
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess && dev < 64) devices.fetch_or(bit, std::memory_order_relaxed);
-    return e;
-}
-
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -722,9 +711,6 @@ __global__ void __launch_bounds__(kThreads, kTraverseCtas) traverse_kernel(const
 // Launch of one instantiation of the extraction.
 template <int FT, int MODE, class UF, bool EXTRA>
 inline cudaError_t launch_traverse_kernel(const Volume& V, const TraverseOut& O, int grid, cudaStream_t st) {
-    static std::atomic<uint64_t> devices{0};
-    const cudaError_t e = allow_traverse_smem(traverse_kernel<FT, MODE, UF, EXTRA>, kTraverseSmem, devices);
-    if (e != cudaSuccess) return e;
     return launch_dependent(traverse_kernel<FT, MODE, UF, EXTRA>, grid, kThreads, kTraverseSmem, st, V, O);
 }
 

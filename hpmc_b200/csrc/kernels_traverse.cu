@@ -476,12 +476,10 @@ static cudaError_t launch_mesh_vertices(const Volume& V, const MeshIO& M, int mo
 
 cudaError_t launch_mesh(const Volume& V, const MeshIO& M, int normal_mode, int traverse_grid, int grid,
                         cudaStream_t st) {
-    static std::atomic<uint64_t> devices{0};
-    cudaError_t e = allow_traverse_smem(mesh_edges, kTraverseSmem, devices);
-    if (e != cudaSuccess || M.count == 0) return e;
+    if (M.count == 0) return cudaSuccess;
     const int mode = V.binary ? kModeBinary : (normal_mode == kNormalsCentral ? kModeCentral : kModeForward);
     const unsigned int tiles = ((M.count + 31u) / 32u + kScanTile - 1) / kScanTile;
-    e = launch_dependent(mesh_edges, traverse_grid, kThreads, kTraverseSmem, st, V, M);
+    cudaError_t e = launch_dependent(mesh_edges, traverse_grid, kThreads, kTraverseSmem, st, V, M);
     if (e == cudaSuccess) e = launch_dependent(mesh_insert, grid, kThreads, 0, st, M, V.ctrl);
     if (e == cudaSuccess) e = launch_dependent(mesh_mark, grid, kThreads, 0, st, M, V.ctrl);
     if (e == cudaSuccess) e = launch_dependent(mesh_scan, tiles, kThreads, 0, st, M, V.ctrl);
@@ -526,9 +524,6 @@ cudaError_t launch_traverse(const Volume& V, const TraverseOut& O, int normal_mo
 
 template <int FT, int MODE>
 static cudaError_t launch_adjoint_kernel(const Volume& V, const AdjointIO& A, int grid, cudaStream_t st) {
-    static std::atomic<uint64_t> devices{0};
-    const cudaError_t e = allow_traverse_smem(adjoint_kernel<FT, MODE>, kTraverseSmem, devices);
-    if (e != cudaSuccess) return e;
     adjoint_kernel<FT, MODE><<<grid, kThreads, kTraverseSmem, st>>>(V, A);
     return cudaGetLastError();
 }
@@ -552,9 +547,6 @@ cudaError_t launch_adjoint(const Volume& V, const AdjointIO& A, int normal_mode,
 
 template <int FT, int MODE>
 static cudaError_t launch_batch_kernel(const BatchDev& B, const TraverseOut& O, int grid, cudaStream_t st) {
-    static std::atomic<uint64_t> devices{0};
-    const cudaError_t e = allow_traverse_smem(traverse_batch<FT, MODE>, kBatchSmem, devices);
-    if (e != cudaSuccess) return e;
     traverse_batch<FT, MODE><<<grid, kThreads, kBatchSmem, st>>>(B, O);
     return cudaGetLastError();
 }
@@ -580,10 +572,8 @@ cudaError_t launch_traverse_batch(const BatchDev& B, const TraverseOut& O, int f
 // Resident CTAs per SM of one kernel with `bytes` of dynamic shared memory.
 template <class K>
 static int resident_ctas(K* kernel, size_t bytes) {
-    static std::atomic<uint64_t> devices{0};
     int n = 0;
-    if (allow_traverse_smem(kernel, bytes, devices) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kThreads, bytes) != cudaSuccess || n < 1)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kThreads, bytes) != cudaSuccess || n < 1)
         n = 1;
     return n;
 }
