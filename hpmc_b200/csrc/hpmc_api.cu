@@ -553,7 +553,8 @@ void HPMCbuildHistopyramid(HPMCHistoPyramid* h, GLfloat threshold) {
 GLuint HPMCacquireNumberOfVertices(HPMCHistoPyramid* h) {
     if (!valid(h) || h->broken) return 0;  // hpiface.cpp:296-298
     if (!h->built) return 0;               // init.cpp:146-147: count starts at zero
-    if (!h->count_valid) {
+    // every replay of a captured build may change the count without a call here
+    if (!h->count_valid || h->captured) {
         Ctrl c;
         if (!read_count(h, &c)) {
             set_error(h, HPMC_ERR_CUDA, true);
@@ -735,7 +736,9 @@ int HPMCextractVerticesToBuffers(HPMCTraversalHandle* th, float* pos, float* nrm
             return HPMC_ERR_CUDA;
         }
         *n_written = (uint32_t)std::min<unsigned long long>(c.total, cap);  // what the traversal writes
-        if (c.total > cap) st = HPMC_ERR_CAPACITY;
+        // (the launch went by the last count read, which replays outdate)
+        if (st == HPMC_ERR_CAPACITY && c.total <= cap) th->h->status = HPMC_OK;
+        st = c.total > cap ? HPMC_ERR_CAPACITY : HPMC_OK;
     }
     return st;
 }

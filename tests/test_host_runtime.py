@@ -1,0 +1,89 @@
+"""The library's host code on a stand-in for the CUDA runtime (fake_cudart.c):
+what it believes about the device after replays, failed allocations, failed
+launches and a context reset.  Each case runs in a process of its own."""
+from __future__ import annotations
+
+import ctypes as C
+import os
+import shutil
+import subprocess
+import sys
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+
+
+class Total(C.Structure):  # the head of the control block (hpmc_device.cuh)
+    _fields_ = [("total", C.c_ulonglong), ("reduce_done", C.c_uint), ("status", C.c_uint)]
+
+
+def _handle(L, size=(40, 40, 40)):
+    c = L.HPMCcreateConstants(4, 3)
+    h = L.HPMCcreateHistoPyramid(c)
+    L.HPMCsetLatticeSize(h, *size)
+    field = C.create_string_buffer(4 * size[0] * size[1] * size[2] + 16)
+    assert L.HPMCsetFieldDevice(h, (C.addressof(field) + 15) // 16 * 16, 0, 0, 0) == 0
+    p = C.c_void_p()
+    assert L.HPMCgetDeviceVertexCount(h, C.byref(p)) == 0
+    return c, h, field, C.cast(p, C.POINTER(Total))[0]
+
+
+def case_count_of_replays(L):
+    """Every replay of a captured build may change the count."""
+    _, h, field, ctrl = _handle(L)
+    L.HPMCbuildHistopyramid(h, 0.0)
+    L.fake_capture(1, None)
+    L.HPMCbuildHistopyramid(h, 0.0)
+    L.fake_capture(0, None)
+    th = L.HPMCcreateTraversalHandle(h)
+    for n in (300, 90, 600):
+        ctrl.total = n  # a replay
+        assert L.HPMCacquireNumberOfVertices(h) == n
+        ctrl.total = n + 3  # another one
+        nv, ni = C.c_uint64(), C.c_uint64()
+        assert L.HPMCextractVerticesIndexed(th, None, None, 1 << 20, None, 1 << 20, C.byref(nv), C.byref(ni)) == 0
+        assert ni.value == n + 3
+        ctrl.total = n - 30  # and one whose vertices fit
+        assert L.HPMCextractVerticesToBuffers(th, 16, None, n, C.byref(nv)) == 0
+        assert nv.value == n - 30
+
+
+CASES = {k[5:]: v for k, v in list(globals().items()) if k.startswith("case_")}
+
+
+@pytest.fixture(scope="module")
+def fake_library(hpmc, tmp_path_factory):
+    from hpmc_b200 import build as B
+
+    if not shutil.which("gcc"):
+        pytest.skip("no C compiler")
+    B.build()
+    out = tmp_path_factory.mktemp("fake")
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(B.nvcc())))
+    fake, lib = str(out / "fake_cudart.o"), str(out / "libhpmc_fake.so")
+    subprocess.run(["gcc", "-O1", "-fPIC", "-I" + os.path.join(cuda, "include"), "-c",
+                    os.path.join(HERE, "fake_cudart.c"), "-o", fake], check=True)
+    objs = sorted(os.path.join(B.OBJ_DIR, os.path.basename(s)[:-3] + ".o") for s in B._sources())
+    subprocess.run([B.nvcc(), *B.NVCC_FLAGS[:2], "-shared", "-cudart", "none", "-Xlinker", "-Bsymbolic", "-o", lib,
+                    *objs, fake], check=True)
+    return lib
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_host_runtime(fake_library, name):
+    r = subprocess.run([sys.executable, os.path.abspath(__file__), fake_library, name], capture_output=True, text=True,
+                       cwd=ROOT, timeout=120)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+if __name__ == "__main__":
+    sys.path.insert(0, ROOT)
+    from hpmc_b200 import _capi
+
+    _capi.LIB_PATH = sys.argv[1]
+    lib = _capi.lib()
+    lib.fake_capture.argtypes = [C.c_int, C.c_void_p]
+    lib.fake_limit.argtypes = [C.c_size_t]
+    CASES[sys.argv[2]](lib)
