@@ -784,11 +784,11 @@ int HPMCextractVerticesIndexed(HPMCTraversalHandle* th, float* positions, float*
     // about six, so the table is at most a third full off the grid's boundary.
     size_t tsize = 1;
     while (tsize < (size_t)n + 2) tsize <<= 1;
-    const size_t words = ((size_t)n + 31) / 32;
+    const size_t words = ((size_t)n + 31) / 32, edges = (size_t)n + hpmc::kMeshSpareEdges;
     auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
-    const size_t o_keys = 0, o_tkeys = up(o_keys + 8 * (size_t)n), o_vertex = up(o_tkeys + 12 * tsize),
-                 o_first = up(o_vertex + 4 * (size_t)n), o_place = up(o_first + 4 * (size_t)n),
-                 o_bits = up(o_place + 4 * (size_t)n), o_scan = up(o_bits + 4 * words), o_tiles = up(o_scan + 4 * words),
+    const size_t o_keys = 0, o_tkeys = up(o_keys + 8 * edges), o_vertex = up(o_tkeys + 12 * tsize),
+                 o_first = up(o_vertex + 4 * (size_t)n), o_place = up(o_first + 4 * edges),
+                 o_bits = up(o_place + 4 * edges), o_scan = up(o_bits + 4 * words), o_tiles = up(o_scan + 4 * words),
                  o_meta = up(o_tiles + 4 * ((size_t)n / 65536 + 2)), o_unique = up(o_meta + 2 * (size_t)n),
                  bytes = o_unique + 256;
     if (!th->mesh_mem || th->mesh_cap < bytes) {
@@ -807,6 +807,7 @@ int HPMCextractVerticesIndexed(HPMCTraversalHandle* th, float* positions, float*
     unsigned char* m = th->mesh_mem;
     hpmc::MeshIO M{};
     M.count = n;
+    M.edges = (uint32_t)std::min<size_t>(edges, 0xffffffffu);
     M.keys = reinterpret_cast<unsigned long long*>(m + o_keys);
     M.table_keys = reinterpret_cast<unsigned long long*>(m + o_tkeys);
     M.vertex = reinterpret_cast<uint32_t*>(m + o_vertex);

@@ -56,14 +56,20 @@ struct BatchDev {
 };
 
 // Indexed-mesh extraction: scratch and outputs (device).  An "edge" below is a
-// distinct edge of one group of cells of the traversal (at most `count` in all);
-// its number of listed edges is Ctrl::mesh_edges.
+// distinct edge of one group of cells of the traversal; the number of listed
+// edges is Ctrl::mesh_edges.  Every edge has a vertex of its group, so a build
+// of `count` vertices lists at most that many; where the device's total is
+// larger (the build was replayed after its count was read), the first `count`
+// vertices are welded, and the cell they end in lists at most 12 edges that
+// only later vertices lie on.
+constexpr uint32_t kMeshSpareEdges = 16;
 struct MeshIO {
     uint32_t count;                  // soup vertices (the vertex count of the build)
+    uint32_t edges;                  // entries for edges: count + kMeshSpareEdges; none is listed past them
     uint32_t* vertex;                // count: edge of each soup vertex
     uint16_t* meta;                  // count: case | vertex-in-cell << 8 (binary fields only)
     unsigned long long* keys;        // per edge: mesh_key
-    uint32_t* first;                 // per edge: its smallest soup index in the group
+    uint32_t* first;                 // per edge: its smallest soup index in the group (~0: none below count)
     uint32_t* place;                 // per edge: table slot, then number of its vertex
     unsigned long long* table_keys;  // table_mask + 1 (> count, power of two)
     uint32_t* table_vals;            // right behind table_keys

@@ -300,12 +300,19 @@ struct MeshEdges {
         }
         __syncwarp();
         for (uint32_t i = (uint32_t)G.lane; i < G.nedges; i += 32) {
+            if (j0 + i >= M.edges) break;
             M.keys[j0 + i] = key[i];
             M.first[j0 + i] = first[i];
         }
         __syncwarp();
     }
 };
+
+// The listed edges.
+__device__ __forceinline__ uint32_t listed_edges(const MeshIO& M, const Ctrl* ctrl) {
+    const uint32_t n = __ldcg(&ctrl->mesh_edges);
+    return n < M.edges ? n : M.edges;
+}
 
 __global__ void __launch_bounds__(kThreads, kTraverseCtas) mesh_edges(const __grid_constant__ Volume V,
                                                                       const __grid_constant__ MeshIO M) {
@@ -342,8 +349,12 @@ __device__ __forceinline__ uint32_t key_hash(unsigned long long k) {
 __global__ void __launch_bounds__(kThreads) mesh_insert(const __grid_constant__ MeshIO M, Ctrl* ctrl) {
     wait_prior_grid();
     allow_next_grid();
-    const uint32_t n = __ldcg(&ctrl->mesh_edges);
+    const uint32_t n = listed_edges(M, ctrl);
     for (uint32_t j = blockIdx.x * kThreads + threadIdx.x; j < n; j += gridDim.x * kThreads) {
+        if (M.first[j] >= M.count) {  // only vertices past the count lie on it
+            M.place[j] = 0xffffffffu;
+            continue;
+        }
         const unsigned long long key = M.keys[j];
         uint32_t h = key_hash(key) & M.table_mask, place = 0xffffffffu;
         for (uint32_t probe = 0; probe <= M.table_mask; probe++) {  // the table has more slots than keys
@@ -363,10 +374,10 @@ __global__ void __launch_bounds__(kThreads) mesh_insert(const __grid_constant__ 
 __global__ void __launch_bounds__(kThreads) mesh_mark(const __grid_constant__ MeshIO M, Ctrl* ctrl) {
     wait_prior_grid();
     allow_next_grid();
-    const uint32_t n = __ldcg(&ctrl->mesh_edges);
+    const uint32_t n = listed_edges(M, ctrl);
     for (uint32_t j = blockIdx.x * kThreads + threadIdx.x; j < n; j += gridDim.x * kThreads) {
         const uint32_t h = M.place[j], f = M.first[j];
-        if (h <= M.table_mask && M.table_vals[h] == f) atomicOr(&M.bits[f >> 5], 1u << (f & 31u));
+        if (f < M.count && h <= M.table_mask && M.table_vals[h] == f) atomicOr(&M.bits[f >> 5], 1u << (f & 31u));
     }
 }
 
@@ -435,11 +446,12 @@ __global__ void __launch_bounds__(kThreads) mesh_vertices(const __grid_constant_
                                                           const __grid_constant__ MeshIO M) {
     wait_prior_grid();
     allow_next_grid();
-    const uint32_t n = __ldcg(&V.ctrl->mesh_edges);
+    const uint32_t n = listed_edges(M, V.ctrl);
     for (uint32_t j = blockIdx.x * kThreads + threadIdx.x; j < n; j += gridDim.x * kThreads) {
         const uint32_t h = M.place[j];
-        if (h > M.table_mask) continue;  // not inserted: reported there
+        if (h > M.table_mask) continue;  // not inserted
         const uint32_t f = M.table_vals[h], word = f >> 5;
+        if (f >= M.count) continue;
         const uint32_t u = M.tile_sums[word / kScanTile] + M.scan[word] +
                            (uint32_t)__popc(M.bits[word] & ((1u << (f & 31u)) - 1u));
         M.place[j] = u;
@@ -462,9 +474,13 @@ __global__ void __launch_bounds__(kThreads) mesh_indices(const __grid_constant__
     wait_prior_grid();
     if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->mesh_edges = 0;
     if (!M.indices) return;
-    const uint32_t n = (uint32_t)(M.icap < M.count ? M.icap : M.count);
-    for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads)
-        M.indices[i] = M.place[M.vertex[i]];
+    // (vertices past the total were not listed)
+    const unsigned long long total = ctrl->total < M.count ? ctrl->total : M.count;
+    const uint32_t n = (uint32_t)(M.icap < total ? M.icap : total);
+    for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
+        const uint32_t j = M.vertex[i];
+        M.indices[i] = j < M.edges ? M.place[j] : 0xffffffffu;
+    }
 }
 
 template <int FT>
