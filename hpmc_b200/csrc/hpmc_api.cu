@@ -211,6 +211,8 @@ bool setup(HPMCHistoPyramid* h) {
     std::memcpy(h->layout, L, sizeof L);
     Volume& V = h->V;
     V = Volume{};
+    // whatever fails from here on, there is no pyramid and no count to be read
+    h->built = h->count_valid = h->host_written = false;
     long long levels_total = 0, slots = 0;
     hpmc::host::volume_layout(V, h->lattice, h->cells, h->extent, L, &levels_total, &slots);
     V.column_slices = hpmc::host::default_column_slices(V, h->constants->num_sms);
@@ -251,8 +253,6 @@ bool setup(HPMCHistoPyramid* h) {
     V.ctrl = h->d_ctrl;
     h->set = 0;
     h->tainted = false;
-    h->built = false;
-    h->count_valid = false;
     return true;
 }
 

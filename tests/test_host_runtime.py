@@ -50,6 +50,32 @@ def case_count_of_replays(L):
         assert nv.value == n - 30
 
 
+def case_failed_setup(L):
+    """A set-up that ran out of memory leaves nothing that could be read or extracted."""
+    for size in ((400, 400, 400), (40, 40, 40)):  # the larger pyramid, then a smaller one
+        _, h, field, ctrl = _handle(L)
+        th = L.HPMCcreateTraversalHandle(h)
+        L.HPMCbuildHistopyramid(h, 0.0)
+        L.HPMCsetLatticeSize(h, 400, 400, 400)
+        L.fake_limit(1 << 16)
+        L.HPMCbuildHistopyramid(h, 0.0)
+        L.fake_limit(1 << 30)
+        assert L.HPMCgetLastError(h) == 6  # HPMC_ERR_OUT_OF_MEMORY
+        launches = L.fake_launches()
+        assert L.HPMCacquireNumberOfVertices(h) == 0
+        assert L.HPMCextractVerticesToBuffers(th, 16, None, 1, None) == 8  # HPMC_ERR_NOT_BUILT
+        assert L.HPMCextractVerticesAdjoint(th, None, None, 1, 16) == 8
+        assert L.HPMCextractVerticesIndexed(th, None, None, 0, None, 0, None, None) == 8
+        assert L.HPMCreadLevel(h, 5, 4096, 1 << 20) == 8
+        assert L.fake_launches() == launches
+        L.HPMCsetLatticeSize(h, *size)
+        L.HPMCbuildHistopyramid(h, 0.0)
+        p = C.c_void_p()
+        assert L.HPMCgetDeviceVertexCount(h, C.byref(p)) == 0
+        assert L.HPMCextractVerticesToBuffers(th, 16, None, 1, None) == 0
+        assert L.HPMCgetLastError(h) == 0
+
+
 CASES = {k[5:]: v for k, v in list(globals().items()) if k.startswith("case_")}
 
 
