@@ -99,6 +99,8 @@ struct HPMCHistoPyramid {
     // whose replays may run on any stream and after other builds
     cudaStream_t build_stream = nullptr;
     bool captured = false;
+    // a weld failed part-way: its counters in the control block are not zero
+    bool weld_failed = false;
     // the last extraction's outputs (byte ranges), stream and set: the next
     // build overlaps it only on the same stream, into the other set, and with
     // a field that is none of those outputs
@@ -826,12 +828,18 @@ int HPMCextractVerticesIndexed(HPMCTraversalHandle* th, float* positions, float*
     M.indices = indices;
     M.icap = index_capacity;
     const int grid = h->constants->num_sms * 8;
-    cudaError_t e = hpmc::launch_mesh(h->V, M, h->normal_mode, traverse_grid(h), grid, h->stream);
+    cudaError_t e = cudaSuccess;
+    if (h->weld_failed) {
+        static_assert(offsetof(Ctrl, mesh_done) == offsetof(Ctrl, mesh_edges) + sizeof(unsigned int), "cleared together");
+        e = cudaMemsetAsync(&h->d_ctrl->mesh_edges, 0, 2 * sizeof(unsigned int), h->stream);
+    }
+    if (e == cudaSuccess) e = hpmc::launch_mesh(h->V, M, h->normal_mode, traverse_grid(h), grid, h->stream);
     unsigned int unique = 0;
     if (e == cudaSuccess && !h->host)
         e = cudaMemcpyAsync(&unique, M.unique, sizeof unique, cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e == cudaSuccess && h->host) unique = *static_cast<volatile unsigned int*>(&h->host->unique);
+    h->weld_failed = e != cudaSuccess;
     if (e != cudaSuccess) {
         cudaGetLastError();
         set_error(h, HPMC_ERR_CUDA, true);

@@ -16,7 +16,9 @@ ROOT = os.path.dirname(HERE)
 
 
 class Total(C.Structure):  # the head of the control block (hpmc_device.cuh)
-    _fields_ = [("total", C.c_ulonglong), ("reduce_done", C.c_uint), ("status", C.c_uint)]
+    _fields_ = [("total", C.c_ulonglong)] + [(n, C.c_uint) for n in (
+        "reduce_done", "status", "written", "work_next", "work_done", "col_next", "col_done", "extracting",
+        "mesh_edges", "mesh_done")]
 
 
 def _handle(L, size=(40, 40, 40)):
@@ -74,6 +76,24 @@ def case_failed_setup(L):
         assert L.HPMCgetDeviceVertexCount(h, C.byref(p)) == 0
         assert L.HPMCextractVerticesToBuffers(th, 16, None, 1, None) == 0
         assert L.HPMCgetLastError(h) == 0
+
+
+def case_failed_weld(L):
+    """A weld whose launches fail part-way leaves its counters behind; the next one starts from zero."""
+    _, h, field, ctrl = _handle(L)
+    th = L.HPMCcreateTraversalHandle(h)
+    L.HPMCbuildHistopyramid(h, 0.0)
+    L.HPMCbuildHistopyramid(h, 0.0)  # (the count of the first was not read: the second's is copied)
+    ctrl.total = 100
+    weld = lambda: L.HPMCextractVerticesIndexed(th, None, None, 1 << 20, None, 1 << 20, None, None)  # noqa: E731
+    assert weld() == 0
+    for after in range(6):  # mesh_edges .. mesh_indices
+        L.fake_fail_launch(L.fake_launches() + after)
+        assert weld() == 5  # HPMC_ERR_CUDA
+        ctrl.mesh_edges, ctrl.mesh_done = 70, 1
+        assert L.HPMCsetFieldDevice(h, 16, 0, 0, 0) == 0  # un-breaks the handle without a set-up
+        assert weld() == 0
+        assert (ctrl.total, ctrl.mesh_edges, ctrl.mesh_done) == (100, 0, 0)
 
 
 CASES = {k[5:]: v for k, v in list(globals().items()) if k.startswith("case_")}
