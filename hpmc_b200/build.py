@@ -33,7 +33,6 @@ NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
-    "--expt-relaxed-constexpr",
     "-I" + os.path.join(ROOT, "include"), "-I" + CSRC,
 ]
 

@@ -34,20 +34,20 @@ enum { kModeForward = kGeomForward, kModeCentral = kGeomCentral, kModeBinary = k
 namespace {
 
 // Edges of a cell by axis and the offset (sx, sy, sz) of their lower end.
-constexpr uint32_t edge_geometry(int e) { return (uint32_t)(kEdgeGeometry >> (5 * e)) & 31u; }
-constexpr int edge_id(int axis, int sx, int sy, int sz) {
+__host__ __device__ constexpr uint32_t edge_geometry(int e) { return (uint32_t)(kEdgeGeometry >> (5 * e)) & 31u; }
+__host__ __device__ constexpr int edge_id(int axis, int sx, int sy, int sz) {
     for (int e = 0; e < 12; e++)
         if (edge_geometry(e) == (uint32_t)(sx | (sy << 1) | (sz << 2) | (axis << 3))) return e;
     return 12;
 }
 // Edges with lower end at offset sx = 1 (sy = 1), and below edge e.
-constexpr uint32_t edges_at(int bit) {
+__host__ __device__ constexpr uint32_t edges_at(int bit) {
     uint32_t m = 0;
     for (int e = 0; e < 12; e++) m |= ((edge_geometry(e) >> bit) & 1u) << e;
     return m;
 }
 constexpr uint32_t kRightEdges = edges_at(0), kUpperEdges = edges_at(1);
-constexpr uint32_t below_edge(int e) { return (1u << e) - 1u; }
+__host__ __device__ constexpr uint32_t below_edge(int e) { return (1u << e) - 1u; }
 
 constexpr int kWindowCells = 32;   // active cells a warp works on at a time (one per lane)
 constexpr int kWindowEdges = 96;   // distinct edges of a window (8 cells never have more)
