@@ -60,6 +60,10 @@ class Layout:
         return 1 if e <= 0 else 1 << (2 * e)
 
 
+class ReferenceHarnessMissing(RuntimeError):
+    """No compiled reference harness, and no HPMC source tree to build it from."""
+
+
 _lib = None
 _ref = None
 
@@ -108,7 +112,11 @@ def ref():
     if _ref is None:
         path = os.path.join(_REF_DIR, "libhpmc_ref.so")
         if not os.path.exists(path):
-            raise RuntimeError(f"reference harness not built: {path} missing")
+            from hpmc_b200.build import DEFAULT_HPMC_SRC
+
+            tree = os.environ.get("HPMC_SRC", DEFAULT_HPMC_SRC)
+            have_tree = os.path.exists(os.path.join(tree, "hpmc", "src", "tables.cpp"))
+            raise (RuntimeError if have_tree else ReferenceHarnessMissing)(f"reference harness not built: {path} missing")
         R = C.CDLL(path)
         ip = C.POINTER(C.c_int)
         R.hpmc_ref_layout.argtypes = [C.c_int] * 6 + [ip]

@@ -16,6 +16,17 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "slow: full-size workloads")
 
 
+@pytest.hookimpl(wrapper=True)
+def pytest_runtest_call(item):
+    """A test that needs the reference's own code is skipped where there is no HPMC tree to compile it from."""
+    from oracle.oracle import ReferenceHarnessMissing
+
+    try:
+        return (yield)
+    except ReferenceHarnessMissing as e:
+        pytest.skip(f"{e}, and no HPMC source tree")
+
+
 @pytest.fixture(scope="session")
 def oracle():
     """The CPU oracle (built from oracle/Makefile; needs the HPMC tree only to build)."""
