@@ -89,11 +89,12 @@ struct HPMCHistoPyramid {
     int nsets = 0;
     int set = 0;                   // the set of the last build
     Ctrl* d_ctrl = nullptr;
-    // where builds leave their count (mapped host memory), or null.  A build
-    // writes it when the count of the build before was read: the write holds up
-    // the end of the reduction by about 1 us, which a loop that never reads the
-    // count need not pay.
+    // where builds leave their count (mapped host memory, 3.5 us to allocate and
+    // free), or null: then it is copied.  A build writes it when the count of the
+    // build before was read: the write holds up the end of the reduction by about
+    // 1 us, which a loop that never reads the count need not pay.
     hpmc::HostCount* host = nullptr;
+    unsigned long long host_context = 0;  // the context it lives in
     bool count_read = true, host_written = false;
     // the last build's stream; whether a build was ever captured into a graph,
     // whose replays may run on any stream and after other builds
@@ -149,11 +150,16 @@ void set_error(HPMCHistoPyramid* h, int status, bool brk) {
     if (brk) h->broken = true;
 }
 
+// The handle's host memory, if the context that it lives in is still there.
+hpmc::HostCount* host_count(const HPMCHistoPyramid* h) {
+    return h->host && h->host_context == hpmc::host::context_id() ? h->host : nullptr;
+}
+
 void release_device(HPMCHistoPyramid* h) {
     cudaFree(h->d_levels);
     cudaFree(h->d_arena);
     cudaFree(h->d_ctrl);
-    hpmc::host::give_host_slot(h->host);
+    if (h->host) cudaFreeHost(h->host);
     h->host = nullptr;
     h->d_levels = nullptr;
     h->d_arena = nullptr;
@@ -236,8 +242,12 @@ bool setup(HPMCHistoPyramid* h) {
             h->status = HPMC_ERR_OUT_OF_MEMORY;
             return false;
         }
-        static_assert(sizeof(hpmc::HostCount) <= 64, "a host slot holds it");
-        h->host = static_cast<hpmc::HostCount*>(hpmc::host::take_host_slot());
+        if (cudaHostAlloc(reinterpret_cast<void**>(&h->host), sizeof(hpmc::HostCount),
+                          cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+            cudaGetLastError();
+            h->host = nullptr;
+        }
+        h->host_context = hpmc::host::context_id();
         h->levels_cap = (size_t)levels_total;
         h->arena_cap = arena_words;
         h->nsets = nsets;
@@ -311,13 +321,13 @@ int launch_extract(HPMCTraversalHandle* th, float* pos, float* nrm, float* feedb
 // reads them the build's last reduction has written them to mapped host memory
 // (the copy this replaces cost about 10 us a call).  After a build on another
 // stream or in a captured graph, the copy, which also waits for the default
-// stream's work and reads what ran last.
+// stream's work and reads what ran last; and in a context that a reset ended,
+// where it fails.
 bool read_count(HPMCHistoPyramid* h, Ctrl* c) {
     if (cudaStreamSynchronize(h->stream) != cudaSuccess) return false;
     h->count_read = true;
-    if (!h->host_written || h->build_stream != h->stream)
-        return cudaMemcpy(c, h->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost) == cudaSuccess;
-    const volatile hpmc::HostCount* s = h->host;
+    const volatile hpmc::HostCount* s = h->host_written && h->build_stream == h->stream ? host_count(h) : nullptr;
+    if (!s) return cudaMemcpy(c, h->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost) == cudaSuccess;
     c->total = s->total;
     c->status = s->status;
     return true;
@@ -566,7 +576,7 @@ GLuint HPMCacquireNumberOfVertices(HPMCHistoPyramid* h) {
             // reported once: the next build starts from a clean status word
             // (the handle may be un-broken by a setter that does not taint)
             cudaMemsetAsync(&h->d_ctrl->status, 0, sizeof(unsigned int), h->stream);
-            if (h->host) h->host->status = 0;
+            if (hpmc::HostCount* s = host_count(h)) s->status = 0;
         }
         if (c.status & hpmc::kStatusTimeout) {
             set_error(h, HPMC_ERR_TIMEOUT, true);
@@ -939,7 +949,7 @@ int HPMCgetDeviceStatus(HPMCHistoPyramid* h, unsigned int* status) {
     *status = c.status;
     const unsigned int zero = 0;
     cudaMemcpy(&h->d_ctrl->status, &zero, sizeof zero, cudaMemcpyHostToDevice);
-    if (h->host) h->host->status = 0;
+    if (hpmc::HostCount* s = host_count(h)) s->status = 0;
     return HPMC_OK;
 }
 

@@ -94,6 +94,7 @@ struct HPMCBatch {
     // status and offsets of the last extraction in mapped host memory (null for
     // very many volumes, whose offsets are copied when they are asked for)
     unsigned long long* host = nullptr;
+    unsigned long long host_context = 0;  // the context it lives in
     bool extracted = false;
 };
 
@@ -109,7 +110,7 @@ void release(HPMCBatch* b) {
     b->capture_stream = nullptr;
     cudaFree(b->d_base);
     b->d_base = nullptr;
-    cudaFreeHost(b->host);
+    if (b->host) cudaFreeHost(b->host);
     b->host = nullptr;
 }
 
@@ -401,6 +402,7 @@ int HPMCcreateBatch(HPMCConstants* c, const HPMCBatchVolume* volumes, int count,
         cudaGetLastError();
         b->host = nullptr;
     }
+    b->host_context = hpmc::host::context_id();
     b->d_bctrl = reinterpret_cast<BatchCtrl*>(b->d_base + o_bctrl);
     b->d_ctrls = reinterpret_cast<Ctrl*>(b->d_base + o_ctrls);
     uint32_t* d_levels = reinterpret_cast<uint32_t*>(b->d_base + o_levels);
@@ -502,7 +504,7 @@ int HPMCbatchGetOffsets(HPMCBatch* b, unsigned long long* host_offsets) {
     if (!valid(b)) return HPMC_ERR_INVALID_HANDLE;
     if (!host_offsets) return HPMC_ERR_INVALID_VALUE;
     BatchCtrl bc;
-    if (b->host && b->extracted) {
+    if (b->host && b->extracted && b->host_context == hpmc::host::context_id()) {
         if (cudaStreamSynchronize(b->last_stream) != cudaSuccess) {
             cudaGetLastError();
             return HPMC_ERR_CUDA;

@@ -3,8 +3,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <mutex>
-#include <vector>
 
 namespace hpmc {
 namespace host {
@@ -52,39 +50,20 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
-namespace {
-constexpr size_t kHostSlotBytes = 64, kHostPageBytes = 4096;
-constexpr int kHostPages = 64;  // at most 4096 slots
-std::mutex g_slots_mu;
-std::vector<void*>& free_slots() {
-    static auto* v = new std::vector<void*>;  // (handles may be destroyed after static objects)
-    return *v;
-}
-int g_host_pages = 0;
-}  // namespace
-
-void* take_host_slot() {
-    std::lock_guard<std::mutex> lk(g_slots_mu);
-    auto& slots = free_slots();
-    if (slots.empty()) {
-        void* page = nullptr;
-        if (g_host_pages >= kHostPages) return nullptr;
-        if (cudaHostAlloc(&page, kHostPageBytes, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+unsigned long long context_id() {
+    using GetId = CUresult (*)(CUcontext, unsigned long long*);
+    static const GetId get = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
             cudaGetLastError();
-            return nullptr;
+            p = nullptr;
         }
-        g_host_pages++;
-        for (size_t o = 0; o < kHostPageBytes; o += kHostSlotBytes) slots.push_back(static_cast<char*>(page) + o);
-    }
-    void* s = slots.back();
-    slots.pop_back();
-    return s;
-}
-
-void give_host_slot(void* slot) {
-    if (!slot) return;
-    std::lock_guard<std::mutex> lk(g_slots_mu);
-    free_slots().push_back(slot);
+        return reinterpret_cast<GetId>(p);
+    }();
+    unsigned long long id = 0;
+    return get && get(nullptr, &id) == CUDA_SUCCESS ? id : 0;
 }
 
 void volume_layout(Volume& V, const int lattice[3], const int cells[3], const float extent[3], const int L[6],

@@ -48,12 +48,9 @@ inline int field_type(int scalar_type) {
                                               : kFieldUNorm8;
 }
 
-// 64 bytes of mapped host memory, from a bounded pool of the process that every
-// thread may use (a pinned allocation per handle would cost more than the copy
-// it saves); null when the pool or pinned memory is exhausted, and the callers
-// then copy.  give_host_slot takes it back once nothing on the device writes it.
-void* take_host_slot();
-void give_host_slot(void* slot);
+// The calling thread's current context: another one after cudaDeviceReset, which
+// ends every allocation of the one before.  0 if the driver does not tell.
+unsigned long long context_id();
 
 // Geometry and compact-pyramid members of V from the lattice, the grid and
 // the layout L (everything except the field, the device pointers and iso).

@@ -96,6 +96,22 @@ def case_failed_weld(L):
         assert (ctrl.total, ctrl.mesh_edges, ctrl.mesh_done) == (100, 0, 0)
 
 
+def case_context_reset(L):
+    """Host memory of a context that was reset is neither handed out nor read."""
+    _, h, field, ctrl = _handle(L)
+    L.HPMCbuildHistopyramid(h, 0.0)
+    assert L.HPMCacquireNumberOfVertices(h) == 0
+    L.HPMCdestroyHandle(h)
+    L.fake_new_context()
+    allocs = L.fake_host_allocs()
+    _, h, field, ctrl = _handle(L)
+    assert L.fake_host_allocs() == allocs + 1
+    L.HPMCbuildHistopyramid(h, 0.0)
+    ctrl.total = 50
+    L.fake_new_context()
+    assert L.HPMCacquireNumberOfVertices(h) == 50  # copied, as far as the runtime lets it
+
+
 CASES = {k[5:]: v for k, v in list(globals().items()) if k.startswith("case_")}
 
 
