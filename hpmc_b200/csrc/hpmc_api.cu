@@ -977,6 +977,7 @@ struct StaticDeviceState {
     int num_sms = 0;
     int traverse_ctas_per_sm = 0;
     bool ready = false;
+    unsigned long long context = 0;    // in which that is its address
 };
 
 std::mutex g_static_mu;
@@ -984,7 +985,7 @@ StaticDeviceState g_static_dev[kStaticMaxDevices];
 
 size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 
-// Once per device, with that device current: look up the scratch array's
+// Once per device and context, with that device current: look up the scratch array's
 // device address and configure the kernels.
 int static_device_setup(StaticDeviceState** out) {
     int dev = 0;
@@ -995,7 +996,8 @@ int static_device_setup(StaticDeviceState** out) {
     if (dev < 0 || dev >= kStaticMaxDevices) return HPMC_ERR_UNSUPPORTED;
     std::lock_guard<std::mutex> lk(g_static_mu);
     StaticDeviceState& s = g_static_dev[dev];
-    if (!s.ready) {
+    const unsigned long long context = hpmc::host::context_id();
+    if (!s.ready || s.context != context) {
         void* p = nullptr;
         if (cudaGetSymbolAddress(&p, g_static_scratch) != cudaSuccess || !p) {
             cudaGetLastError();
@@ -1007,6 +1009,7 @@ int static_device_setup(StaticDeviceState** out) {
             return HPMC_ERR_CUDA;
         }
         s.scratch = static_cast<unsigned char*>(p);
+        s.context = hpmc::host::context_id();  // (the first call of a process has made the context by now)
         s.num_sms = prop.multiProcessorCount;
         s.traverse_ctas_per_sm = hpmc::traverse_blocks_per_sm();
         hpmc::column_smem_ok();

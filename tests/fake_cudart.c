@@ -8,7 +8,7 @@
 #include <string.h>
 
 static size_t g_limit = (size_t)1 << 30;
-static int g_launches, g_fail_launch = -1, g_host_allocs, g_syncs;
+static int g_launches, g_fail_launch = -1, g_host_allocs, g_symbols;
 static cudaStream_t g_capturing;
 static int g_any_capture;
 static unsigned long long g_context = 1;
@@ -21,7 +21,7 @@ void fake_capture(int on, void *stream) { g_any_capture = on; g_capturing = (cud
 void fake_new_context(void) { g_context++; }                   /* as after cudaDeviceReset */
 int fake_launches(void) { return g_launches; }
 int fake_host_allocs(void) { return g_host_allocs; }
-int fake_syncs(void) { return g_syncs; }
+int fake_symbol_lookups(void) { return g_symbols; }
 
 /* --- registration ---------------------------------------------------------- */
 void **__cudaRegisterFatBinary(void *f) { (void)f; static void *h; return &h; }
@@ -73,7 +73,7 @@ cudaError_t cudaMemset(void *d, int v, size_t n) {
     return cudaSuccess;
 }
 cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t st) { (void)st; return cudaMemset(d, v, n); }
-cudaError_t cudaGetSymbolAddress(void **p, const void *s) { *p = (void *)s; return cudaSuccess; }
+cudaError_t cudaGetSymbolAddress(void **p, const void *s) { g_symbols++; *p = (void *)s; return cudaSuccess; }
 
 /* --- launches ----------------------------------------------------------------- */
 static cudaError_t launch(void) { return g_launches++ == g_fail_launch ? cudaErrorLaunchOutOfResources : cudaSuccess; }
@@ -109,8 +109,8 @@ cudaError_t cudaGetDriverEntryPoint(const char *name, void **fn, unsigned long l
     if (q) *q = *fn ? cudaDriverEntryPointSuccess : cudaDriverEntryPointSymbolNotFound;
     return *fn ? cudaSuccess : cudaErrorSymbolNotFound;
 }
-cudaError_t cudaDeviceSynchronize(void) { g_syncs++; return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t s) { (void)s; g_syncs++; return cudaSuccess; }
+cudaError_t cudaDeviceSynchronize(void) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { (void)s; return cudaSuccess; }
 cudaError_t cudaStreamIsCapturing(cudaStream_t s, enum cudaStreamCaptureStatus *st) {
     *st = g_any_capture && s == g_capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
     return cudaSuccess;

@@ -112,6 +112,20 @@ def case_context_reset(L):
     assert L.HPMCacquireNumberOfVertices(h) == 50  # copied, as far as the runtime lets it
 
 
+def case_static_scratch_after_reset(L):
+    """The scratch array has an address per context."""
+    field = C.create_string_buffer(4 * 20 * 20 * 20 + 16)
+    count = C.c_uint()
+    lookups = []
+    for _ in range(2):
+        for _ in range(2):
+            assert L.HPMCextractStatic((C.addressof(field) + 15) // 16 * 16, 0, 20, 20, 20, 0, 0, 0.0, 0, None, None, None, 0,
+                                       C.byref(count), None, None) == 0
+        lookups.append(L.fake_symbol_lookups())
+        L.fake_new_context()
+    assert lookups == [1, 2]
+
+
 CASES = {k[5:]: v for k, v in list(globals().items()) if k.startswith("case_")}
 
 
