@@ -377,7 +377,7 @@ HPMCConstants* HPMCcreateConstants(GLint max_gl_major, GLint max_gl_minor) {
     c->device = dev;
     c->num_sms = prop.multiProcessorCount;
     c->traverse_ctas_per_sm = hpmc::traverse_blocks_per_sm();
-    hpmc::column_smem_ok();
+    hpmc::column_smem_opt_in();
     return c;
 }
 
@@ -1012,7 +1012,7 @@ int static_device_setup(StaticDeviceState** out) {
         s.context = hpmc::host::context_id();  // (the first call of a process has made the context by now)
         s.num_sms = prop.multiProcessorCount;
         s.traverse_ctas_per_sm = hpmc::traverse_blocks_per_sm();
-        hpmc::column_smem_ok();
+        hpmc::column_smem_opt_in();
         s.ready = true;
     }
     *out = &s;

@@ -98,7 +98,9 @@ cudaError_t launch_reduce(const Volume& V, cudaStream_t st);
 cudaError_t launch_traverse(const Volume& V, const TraverseOut& O, int normal_mode, int grid,
                             cudaStream_t st);
 cudaError_t launch_adjoint(const Volume& V, const AdjointIO& A, int normal_mode, int grid, cudaStream_t st);
-bool column_smem_ok();
+// The TMA classifiers' dynamic shared memory on the current device: holds until
+// its context is reset, so constants set it up each time they are created.
+void column_smem_opt_in();
 int traverse_blocks_per_sm();
 
 }  // namespace hpmc

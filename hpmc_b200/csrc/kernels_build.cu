@@ -577,7 +577,6 @@ constexpr int kRingBytesU8 = kRingStages * ((48 * 33 * kLayersPerBox + 127) & ~1
 static int column_ctas_per_sm() {
     static int n = 0;
     if (n == 0) {
-        column_smem_ok();
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, classify_columns<kFieldF32>, kThreads,
                                                           kRingBytesF32) !=
                 cudaSuccess ||
@@ -669,20 +668,16 @@ cudaError_t launch_reduce_batch(const BatchDev& B, unsigned int chunks, cudaStre
     return cudaGetLastError();
 }
 
-bool column_smem_ok() {
-    static int configured = 0;
-    if (!configured) {
-        cudaFuncSetAttribute(classify_columns<kFieldF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRingBytesF32);
-        cudaFuncSetAttribute(classify_columns<kFieldU8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRingBytesU8);
-        cudaFuncSetAttribute(classify_columns<kFieldUNorm8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kRingBytesU8);
-        cudaFuncSetAttribute(classify_batch_tma<kFieldF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRingBytesF32);
-        cudaFuncSetAttribute(classify_batch_tma<kFieldU8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRingBytesU8);
-        cudaFuncSetAttribute(classify_batch_tma<kFieldUNorm8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kRingBytesU8);
-        configured = 1;
-    }
-    return true;
+void column_smem_opt_in() {
+    const auto opt_in = [](auto* kernel, int bytes) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    };
+    opt_in(classify_columns<kFieldF32>, kRingBytesF32);
+    opt_in(classify_columns<kFieldU8>, kRingBytesU8);
+    opt_in(classify_columns<kFieldUNorm8>, kRingBytesU8);
+    opt_in(classify_batch_tma<kFieldF32>, kRingBytesF32);
+    opt_in(classify_batch_tma<kFieldU8>, kRingBytesU8);
+    opt_in(classify_batch_tma<kFieldUNorm8>, kRingBytesU8);
 }
 
 }  // namespace hpmc

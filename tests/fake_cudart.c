@@ -8,7 +8,7 @@
 #include <string.h>
 
 static size_t g_limit = (size_t)1 << 30;
-static int g_launches, g_fail_launch = -1, g_host_allocs, g_symbols;
+static int g_launches, g_fail_launch = -1, g_host_allocs, g_symbols, g_attributes;
 static cudaStream_t g_capturing;
 static int g_any_capture;
 static unsigned long long g_context = 1;
@@ -22,6 +22,7 @@ void fake_new_context(void) { g_context++; }                   /* as after cudaD
 int fake_launches(void) { return g_launches; }
 int fake_host_allocs(void) { return g_host_allocs; }
 int fake_symbol_lookups(void) { return g_symbols; }
+int fake_attributes(void) { return g_attributes; }
 
 /* --- registration ---------------------------------------------------------- */
 void **__cudaRegisterFatBinary(void *f) { (void)f; static void *h; return &h; }
@@ -85,7 +86,11 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void
     (void)c; (void)f; (void)a;
     return launch();
 }
-cudaError_t cudaFuncSetAttribute(const void *f, enum cudaFuncAttribute a, int v) { (void)f; (void)a; (void)v; return cudaSuccess; }
+cudaError_t cudaFuncSetAttribute(const void *f, enum cudaFuncAttribute a, int v) {
+    (void)f; (void)a; (void)v;
+    g_attributes++;
+    return cudaSuccess;
+}
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const void *f, int b, size_t s, unsigned fl) {
     (void)f; (void)b; (void)s; (void)fl;
     *n = 2;

@@ -126,6 +126,17 @@ def case_static_scratch_after_reset(L):
     assert lookups == [1, 2]
 
 
+def case_opt_in_per_device(L):
+    """The classifiers' shared-memory opt-in holds for one device and until a reset: constants renew it."""
+    set_up = []
+    for _ in range(2):
+        before = L.fake_attributes()
+        L.HPMCdestroyConstants(L.HPMCcreateConstants(4, 3))
+        set_up.append(L.fake_attributes() - before)
+        L.fake_new_context()
+    assert set_up[0] == set_up[1] > 0
+
+
 CASES = {k[5:]: v for k, v in list(globals().items()) if k.startswith("case_")}
 
 
