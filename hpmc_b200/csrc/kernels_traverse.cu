@@ -55,6 +55,21 @@ __device__ __forceinline__ void scatter(const Volume& V, float* dfield, const in
 }
 }  // namespace
 
+// The last group may be cut inside a cell: an edge that only vertices past the
+// cut lie on has no cotangent, and 0 times an overflowing derivative is not 0.
+// The first vertex's edge takes its place, once more with no cotangent.  (Where
+// nothing is cut every edge is seen.)  n: the group's vertices; seen: a word per edge.
+static __device__ __noinline__ void drop_unseen_edges(WarpArea& W, uint32_t* seen, uint32_t nedges, uint32_t n, int lane) {
+    static_assert(kWindowEdges <= 32 * 6, "the staging area has a word per edge");
+    for (uint32_t i = (uint32_t)lane; i < nedges; i += 32) seen[i] = 0u;
+    __syncwarp();
+    for (uint32_t i = (uint32_t)lane; i < n; i += 32) seen[W.slot[i]] = 1u;
+    __syncwarp();
+    for (uint32_t i = (uint32_t)lane; i < nedges; i += 32)
+        if (!seen[i]) W.edge[i] = W.edge[W.slot[0]];
+    __syncwarp();
+}
+
 // Every distinct edge of a group of cells is differentiated once: the vertices
 // on it -- the same crossing emitted by neighbouring triangles -- have the same
 // Jacobian, so their cotangents are summed into the edge's slot first.  (Summing
@@ -65,6 +80,7 @@ struct AdjointVertices {
     const AdjointIO& A;
     float (*agg)[6];    // the warp's staging area, one row per lane
     unsigned long long out;
+    uint32_t end;       // vertices differentiated
 
     __device__ __forceinline__ void run(const CellGroup& G) {
         const Volume& V = G.V;
@@ -102,6 +118,7 @@ struct AdjointVertices {
             }
             __syncwarp();
         }
+        if (G.last == end) drop_unseen_edges(W, reinterpret_cast<uint32_t*>(agg), G.nedges, n, G.lane);
         G.edges([&](uint32_t slot, const EdgeAt& E) {
             const int ax = E.axis;
             const float iso = V.iso;
@@ -178,7 +195,7 @@ __global__ void __launch_bounds__(kThreads, kTraverseCtas) adjoint_kernel(const 
     const uint32_t VW = 32u * item_rounds(N, gridDim.x);
     const uint32_t nchunks = (N + VW - 1) / VW;
     set_volume(V, S.warp[warp], lane);
-    AdjointVertices<FT, MODE> p{A, S_agg[warp], V.vertex_base};
+    AdjointVertices<FT, MODE> p{A, S_agg[warp], V.vertex_base, N};
     for (uint32_t chunk = next_chunk(V, lane); chunk < nchunks; chunk = next_chunk(V, lane))
         walk_range(V, S, S.warp[warp], lane, chunk * VW, min(N, (chunk + 1u) * VW), N, p);
     finish_queue(V);
