@@ -89,12 +89,12 @@ struct HPMCHistoPyramid {
     int nsets = 0;
     int set = 0;                   // the set of the last build
     Ctrl* d_ctrl = nullptr;
-    // where builds leave their count (mapped host memory, 3.5 us to allocate and
-    // free), or null: then it is copied.  A build writes it when the count of the
-    // build before was read: the write holds up the end of the reduction by about
-    // 1 us, which a loop that never reads the count need not pay.
+    // where builds leave their count (mapped host memory), or null: then it is
+    // copied.  A build writes it when the count of the build before was read: the
+    // write holds up the end of the reduction by about 1 us, which a loop that
+    // never reads the count need not pay.
     hpmc::HostCount* host = nullptr;
-    unsigned long long host_context = 0;  // the context it lives in
+    hpmc::host::HostSlot host_slot;  // its memory
     bool count_read = true, host_written = false;
     // the last build's stream; whether a build was ever captured into a graph,
     // whose replays may run on any stream and after other builds
@@ -152,14 +152,15 @@ void set_error(HPMCHistoPyramid* h, int status, bool brk) {
 
 // The handle's host memory, if the context that it lives in is still there.
 hpmc::HostCount* host_count(const HPMCHistoPyramid* h) {
-    return h->host && h->host_context == hpmc::host::context_id() ? h->host : nullptr;
+    return h->host && h->host_slot.context == hpmc::host::context_id() ? h->host : nullptr;
 }
 
 void release_device(HPMCHistoPyramid* h) {
     cudaFree(h->d_levels);
     cudaFree(h->d_arena);
     cudaFree(h->d_ctrl);
-    if (h->host) cudaFreeHost(h->host);
+    hpmc::host::give_host_slot(h->host_slot);
+    h->host_slot = {};
     h->host = nullptr;
     h->d_levels = nullptr;
     h->d_arena = nullptr;
@@ -242,12 +243,9 @@ bool setup(HPMCHistoPyramid* h) {
             h->status = HPMC_ERR_OUT_OF_MEMORY;
             return false;
         }
-        if (cudaHostAlloc(reinterpret_cast<void**>(&h->host), sizeof(hpmc::HostCount),
-                          cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
-            cudaGetLastError();
-            h->host = nullptr;
-        }
-        h->host_context = hpmc::host::context_id();
+        static_assert(sizeof(hpmc::HostCount) <= 64, "a host slot holds it");
+        h->host_slot = hpmc::host::take_host_slot();
+        h->host = static_cast<hpmc::HostCount*>(h->host_slot.p);
         h->levels_cap = (size_t)levels_total;
         h->arena_cap = arena_words;
         h->nsets = nsets;

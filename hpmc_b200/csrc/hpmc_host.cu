@@ -3,6 +3,10 @@
 
 #include <algorithm>
 #include <cmath>
+#include <iterator>
+#include <map>
+#include <mutex>
+#include <vector>
 
 namespace hpmc {
 namespace host {
@@ -64,6 +68,54 @@ unsigned long long context_id() {
     }();
     unsigned long long id = 0;
     return get && get(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
+namespace {
+constexpr size_t kHostSlotBytes = 64, kHostPageBytes = 4096;
+constexpr int kHostPages = 64;         // of one context: at most 4096 slots
+constexpr size_t kHostContexts = 64;   // of which slots are kept
+struct HostPool {
+    std::vector<void*> free;
+    int pages = 0;
+};
+std::mutex g_slots_mu;
+std::map<unsigned long long, HostPool>& host_pools() {
+    static auto* m = new std::map<unsigned long long, HostPool>;  // (handles may be destroyed after static objects)
+    return *m;
+}
+}  // namespace
+
+HostSlot take_host_slot() {
+    HostSlot s;
+    s.context = context_id();
+    if (!s.context) return s;
+    std::lock_guard<std::mutex> lk(g_slots_mu);
+    auto& pools = host_pools();
+    HostPool& pool = pools[s.context];
+    if (pools.size() > kHostContexts) {  // the oldest one, most likely long reset (ids only grow)
+        auto oldest = pools.begin();
+        pools.erase(oldest->first == s.context ? std::next(oldest) : oldest);
+    }
+    if (pool.free.empty()) {
+        void* page = nullptr;
+        if (pool.pages >= kHostPages) return s;
+        if (cudaHostAlloc(&page, kHostPageBytes, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+            cudaGetLastError();
+            return s;
+        }
+        pool.pages++;
+        for (size_t o = 0; o < kHostPageBytes; o += kHostSlotBytes) pool.free.push_back(static_cast<char*>(page) + o);
+    }
+    s.p = pool.free.back();
+    pool.free.pop_back();
+    return s;
+}
+
+void give_host_slot(HostSlot slot) {
+    if (!slot.p) return;
+    std::lock_guard<std::mutex> lk(g_slots_mu);
+    auto pool = host_pools().find(slot.context);
+    if (pool != host_pools().end()) pool->second.free.push_back(slot.p);
 }
 
 void volume_layout(Volume& V, const int lattice[3], const int cells[3], const float extent[3], const int L[6],

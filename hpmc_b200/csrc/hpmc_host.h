@@ -52,6 +52,19 @@ inline int field_type(int scalar_type) {
 // ends every allocation of the one before.  0 if the driver does not tell.
 unsigned long long context_id();
 
+// 64 bytes of mapped host memory, from a bounded pool of the context that every
+// thread may use: while another pinned allocation lives one costs 3.5 us, but the
+// first one costs 1.2 to 3.4 ms, which a program with one handle at a time would
+// pay for each.  p is null when the pool or pinned memory is exhausted, and the
+// callers then copy.  give_host_slot takes it back once nothing on the device
+// writes it; a context's slots go with it.
+struct HostSlot {
+    void* p = nullptr;
+    unsigned long long context = 0;
+};
+HostSlot take_host_slot();
+void give_host_slot(HostSlot slot);
+
 // Geometry and compact-pyramid members of V from the lattice, the grid and
 // the layout L (everything except the field, the device pointers and iso).
 // Returns the dense-level entries and the arena slots the volume needs.

@@ -102,8 +102,10 @@ def case_context_reset(L):
     L.HPMCbuildHistopyramid(h, 0.0)
     assert L.HPMCacquireNumberOfVertices(h) == 0
     L.HPMCdestroyHandle(h)
-    L.fake_new_context()
     allocs = L.fake_host_allocs()
+    L.HPMCdestroyHandle(_handle(L)[1])
+    assert L.fake_host_allocs() == allocs == 1  # kept for the next handle ...
+    L.fake_new_context()  # ... of the same context
     _, h, field, ctrl = _handle(L)
     assert L.fake_host_allocs() == allocs + 1
     L.HPMCbuildHistopyramid(h, 0.0)
