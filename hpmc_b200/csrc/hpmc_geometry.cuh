@@ -116,9 +116,9 @@ __device__ __forceinline__ EdgeAt edge_at(const Volume& V, int x, int y, int z, 
 // The field samples one vertex reads: f(a), f(b) with b = a + e_u, f(a - e_u),
 // f(b + e_u), f(a +- e_v), ... -- 12 samples for central differences, 7 forward
 // (f(a + e_u) is f(b), f(b - e_u) is f(a)).  All loads of a vertex are issued
-// in one branch-free block: interior cells through element offsets, boundary
-// cells with each coordinate clamped (GL_CLAMP + NEAREST), functor fields by
-// evaluating the functor.
+// in one branch-free block: interior cells through 32-bit element offsets,
+// boundary cells and fields of 2^31 elements through 64-bit ones that stay inside
+// the lattice (GL_CLAMP + NEAREST), functor fields by evaluating the functor.
 struct EdgeField {
     float va, vb;
     float am, bp;              // f(a - e_u) (central differences only), f(b + e_u)
@@ -158,6 +158,40 @@ __device__ __forceinline__ void gather_edge(const Volume& V, const EdgeAt& E, Ed
             if (CENTRAL) {
                 F.amv[i] = ld(pa - o[i]);
                 F.bmv[i] = ld(pb - o[i]);
+            }
+        }
+    } else if constexpr (kArray) {
+        // One offset per direction from a and from b (both inside the lattice), 0
+        // where it would leave the lattice.  Clamping the three coordinates of each
+        // sample instead costs a 64-bit index per sample and the registers for it:
+        // the byte noise at 256^3 with a slice pitch of 8 MB took 1768 (forward)
+        // and 2088 us (central) instead of 1648 and 1912, the batched traversal
+        // spilled 188 bytes instead of 100 and took 4 to 5 % longer.
+        auto along = [&](auto x, auto y, auto z, int i) {  // component i of (u, v, w)
+            if (i == 0) return E.axis == 0 ? x : E.axis == 1 ? y : z;
+            if (i == 1) return E.axis == 0 ? y : E.axis == 1 ? z : x;
+            return E.axis == 0 ? z : E.axis == 1 ? x : y;
+        };
+        auto step = [&](int i, int d) -> long long {
+            const uint32_t at = (uint32_t)(along(E.a[0], E.a[1], E.a[2], i) + d);
+            const long long stride = along(1ll, V.row_pitch, V.slice_pitch, i);
+            return at < (uint32_t)along(V.lattice[0], V.lattice[1], V.lattice[2], i) ? (d < 0 ? -stride : stride) : 0ll;
+        };
+        const long long pa = (long long)E.a[2] * V.slice_pitch + (long long)E.a[1] * V.row_pitch + E.a[0];
+        const long long su = step(0, 1), pb = pa + su;
+        F.va = fetch_raw<FT>(V, pa);
+        F.vb = fetch_raw<FT>(V, pb);
+        F.bp = fetch_raw<FT>(V, pb + step(0, 2));
+        if (CENTRAL) F.am = fetch_raw<FT>(V, pa + step(0, -1));
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const long long up = step(i + 1, 1);
+            F.ap[i] = fetch_raw<FT>(V, pa + up);
+            F.bpv[i] = fetch_raw<FT>(V, pb + up);
+            if (CENTRAL) {
+                const long long down = step(i + 1, -1);
+                F.amv[i] = fetch_raw<FT>(V, pa + down);
+                F.bmv[i] = fetch_raw<FT>(V, pb + down);
             }
         }
     } else {
