@@ -116,7 +116,8 @@ def ref():
 
             tree = os.environ.get("HPMC_SRC", DEFAULT_HPMC_SRC)
             have_tree = os.path.exists(os.path.join(tree, "hpmc", "src", "tables.cpp"))
-            raise (RuntimeError if have_tree else ReferenceHarnessMissing)(f"reference harness not built: {path} missing")
+            raise (RuntimeError if have_tree else ReferenceHarnessMissing)(
+                f"reference harness not built: {os.path.relpath(path, os.path.dirname(_HERE))} missing")
         R = C.CDLL(path)
         ip = C.POINTER(C.c_int)
         R.hpmc_ref_layout.argtypes = [C.c_int] * 6 + [ip]
