@@ -157,7 +157,7 @@ def derive(tri, edge, mid):
     return count, edge_index, binary_normal
 
 
-def emit(out_path: str, tri, edge, mid) -> None:
+def emit(out_path: str, tri, edge, mid, source: str) -> None:
     count, edge_index, binary_normal = derive(tri, edge, mid)
     packed_edges = 0
     for e in range(12):
@@ -170,7 +170,7 @@ def emit(out_path: str, tri, edge, mid) -> None:
             w |= int(edge_index[c, k]) << (4 * k)
         edge_words.append(w)
     lines = [
-        "// Generated at build time by gen_tables.py from HPMC's hpmc/src/tables.cpp",
+        f"// Generated at build time by gen_tables.py from {source}",
         "// (GPL-2 data of the HPMC project).  Build artefact: not committed, do not edit.",
         "#pragma once",
         "#include <stdint.h>",
@@ -201,7 +201,10 @@ def main(argv):
         print(__doc__)
         return 2
     from_tree = os.path.exists(os.path.join(argv[1], "hpmc", "src", "tables.cpp"))
-    emit(argv[2], *(read_reference_tables if from_tree else read_fixture_tables)(argv[1]))
+    if from_tree:
+        emit(argv[2], *read_reference_tables(argv[1]), "HPMC's hpmc/src/tables.cpp")
+    else:
+        emit(argv[2], *read_fixture_tables(argv[1]), "the golden fixtures")
     return 0
 
 

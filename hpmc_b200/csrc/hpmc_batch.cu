@@ -1,6 +1,6 @@
 // hpmc_batch.cu -- batched extraction: many volumes of uneven lattices and
-// iso-values built, counted and traversed by three launches captured in one
-// CUDA graph.  No counterpart in the reference (it extracts one volume per
+// iso-values built, counted and traversed by three launches (four where some
+// volumes have a tensor map and some have none) captured in one CUDA graph.  No counterpart in the reference (it extracts one volume per
 // HistoPyramid handle, hpmc/include/hpmc.h:330-469); per volume the results
 // equal the handle path's (same layout, same kernels' arithmetic).
 //
@@ -41,7 +41,8 @@ size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // Autotuner choices of this process per batch signature (scalar type, normal
 // mode, SM count and every volume's lattice): a later batch of the same shape
-// takes the choice without timing the 72 candidates again.
+// takes the choice without timing the candidates again (40 where 4 CTAs per SM do
+// not fit).
 std::mutex g_tune_mu;
 std::map<std::vector<long long>, std::array<int, 3>> g_tune_cache;
 

@@ -331,7 +331,8 @@ __device__ __forceinline__ void direct_box_bits(const Volume& V, int x0, int y0,
 // where it is compared.  A layer's four rows are evaluated together (their
 // chains of dependent operations overlap) and the loops around them stay
 // rolled: 35 inlined copies of a functor do not fit the instruction cache
-// (classifier of the cubic at 128^3: 47.4 us unrolled, 16.4 us with one copy).
+// (the cubic at 128^3: 47.4 us unrolled, 16.4 us with one copy in the form of that
+// measurement; 12.9 us now).
 template <int FT, class UF>
 __device__ __forceinline__ void functor_box_bits(const Volume& V, int x0, int y0, int z, int nl, uint32_t gl0, float iso,
                                                  int warp, int lane, ColumnBits& C) {
@@ -369,8 +370,8 @@ __device__ __forceinline__ void functor_box_bits(const Volume& V, int x0, int y0
 // leaves room for 2 CTAs per SM only); functors are evaluated once per sample.  The block
 // classifier it takes over from loads or evaluates 18 samples per 4 cells and
 // visits the padding blocks of the layout.  Kernel times, block classifier ->
-// this one: f32 301x257x129 51.9 -> 17.9 us, UNORM8 253x231x197 62.6 -> 23.7,
-// float4 128^3 18.1 -> 10.5, the cubic functor at 128^3 44.7 -> 14.3.  Issue-
+// this one: f32 301x257x129 51.9 -> 17.9 us, UNORM8 253x231x197 62.6 -> 24.0,
+// float4 128^3 18.1 -> 9.7, the cubic functor at 128^3 44.7 -> 12.9.  Issue-
 // bound on array fields (ballots and slice classification), not by memory.
 //
 // CTA body: column `u` (footprint-fastest) of V.  WAIT: also wait for the

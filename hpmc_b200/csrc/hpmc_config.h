@@ -28,12 +28,17 @@ constexpr int kTopCacheEntries = 344;
 // Resident extraction CTAs per SM (registers; see the note at the kernel).
 constexpr int kTraverseCtas = 3;
 // Rounds of 32 vertices a warp of the single-volume traversal takes at least.
+// Whole calls with 1, 2, 4, 8, us: metaballs 64^3 28.9, 28.8, 28.9, 30.9; cubic
+// functor 128^3 43.9, 43.1, 41.7, 43.3; float4 128^3 39.2, 39.5, 38.3, 39.6; where
+// every warp has more (301x257x129 and up) the same.
 constexpr int kMinRounds = 4;
 // Vertices per warp work item (R rounds of 32) of the batched traversal, until
 // tuned: longer items save descents and part windows, but leave warps without
-// work in a small batch.  8, 16, 32 rounds: 64 volumes of 84 M cells 447, 394,
-// 384 us; 24 of 8 M cells 95, 95, 103.  The single-volume traversal gives each
-// warp one contiguous range instead.
+// work in a small batch.  8, 16, 32 rounds, us, f32 volumes of edge 32..192: 1.7 M
+// cells 39, 46, 62; 5.4 M 63, 61, 81; 16.8 M 97, 97, 106; 27 M 140, 136, 146; 61 M
+// 282, 252, 252; 100 M 421, 372, 365; byte volumes of edge 20..120: 1.3 M 40, 46,
+// 62; 6.4 M 74, 72, 91; 14.7 M 127, 118, 127; 49 M 324, 287, 283.  The single-
+// volume traversal gives each warp one contiguous range instead.
 constexpr int kTraverseRounds = 8;
 constexpr int kLargeBatchRounds = 16;
 constexpr long long kLargeBatchCells = 16ll << 20;

@@ -590,10 +590,11 @@ __device__ __forceinline__ void finish_queue_batch(const BatchDev& Bt) {
 // 3 CTAs of 39 KB leave L1 room for the gathers; 4 (64 registers) measured 1 to
 // 5 % slower, 5 (spills) 5 to 25 %, and a 222 KB footprint of the shared memory
 // 15 % slower on the 512^3 cubic.  kWindowEdges: 96 against 128, the same
-// except the batch, 12 % faster.  Kernel times before -> now: 512^3 cubic 84.5
-// -> 73.0 us, 512x512x33 slab 46.9 -> 34.2, uint8 noise 256^3 360 -> 303,
-// UNORM8 noise 253x231x197 225 -> 163, float4 128^3 28.6 -> 18.5, 64 volumes
-// batched 364 -> 267, metaballs 64^3 24.3 -> 14.4.  UF: a caller's functor type
+// except the batch, 12 % faster.  The batched form spills 52 to 100 bytes at its 80
+// registers, the others nothing.  Kernel times before -> now: 512^3 cubic 84.5
+// -> 72.8 us, 512x512x33 slab 46.9 -> 33.2, uint8 noise 256^3 360 -> 305,
+// UNORM8 noise 253x231x197 225 -> 161, float4 128^3 28.6 -> 18.8, 64 volumes
+// batched 364 -> 247, metaballs 64^3 24.3 -> 14.6.  UF: a caller's functor type
 // when FT == kFieldUser (include/hpmc_functor.cuh).  EXTRA: the interleaved
 // feedback and inspection outputs may be set (false: positions and normals
 // only, without their per-vertex tests).

@@ -330,8 +330,9 @@ int HPMCextractVerticesIndexed(struct HPMCTraversalHandle* th, float* positions,
  *
  * No counterpart in the reference, which builds one volume per HistoPyramid
  * handle.  A batch holds many volumes of uneven lattices and iso-values (one
- * scalar type per batch) and extracts all of them with three launches --
- * classify over every volume's bricks, reduce over every volume's pyramid,
+ * scalar type per batch) and extracts all of them with three or four launches --
+ * classify over every volume's bricks (those that TMA can load, then those that
+ * it cannot), reduce over every volume's pyramid,
  * one persistent traversal -- captured once in a CUDA graph and replayed.
  * Per volume the vertices, their order and their values equal those of
  * HPMCbuildHistopyramid + HPMCextractVerticesToBuffers on that volume.
